@@ -27,7 +27,7 @@ struct tsr_dense {
   int precision = 0;
   int device = 0;
   const float* dX = nullptr;
-  void* owned[2 * tsr::kMaxModes + 4] = {};
+  void* owned[2 * tsr::kMaxModes + 2] = {};
   tsr::ModeOperand ops[tsr::kMaxModes];
   double* d_scalars = nullptr;  // [0] ||X||^2, [1] <X, Xhat>, [2] loss, [3] scratch
   // BF16x3 tensors of 3 or more modes whose trailing-two-modes view
@@ -38,13 +38,10 @@ struct tsr_dense {
   bool d3_three = false;  // the view suits the single-layout 3-way MTTKRP
   bool d3_two = false;    // the view suits the two-sided contraction
   tsr::Dense3 d3{};
-  // FP32 tensors of 3 or more modes: T and P as mode-0 MTTKRPs. vops[0] is X
-  // as the 3-way tensor (A, I_{N-2}, I_{N-1}) (X itself, or a padded copy);
-  // vops[1] is X's transpose (C x A, C = I_{N-2} I_{N-1}) as the tensor
-  // (C, I_0, .., I_{N-3}). Buffers in owned[2N + 2], owned[2N + 3].
+  // FP32 tensors of 3 or more modes: T and P contracted from X seen as an
+  // A x C matrix (A the leading modes' product, C = I_{N-2} I_{N-1})
   bool v2_on = false;
   int64_t v2_shape[2] = {0, 0};
-  tsr::ModeOperand vops[2];
 };
 
 namespace tsr {
@@ -498,6 +495,42 @@ int64_t prod_range(const int64_t* shape, int m0, int m1) {
   return p;
 }
 
+// T (A x R) = X KR(trailing two) and P (C x R) = X^T KR(leading modes) of X
+// seen as A x C (N >= 3 modes, row-major), read in place.
+int contract_sides(tsr_ctx* ctx, const float* dX, int N, const int64_t* shape,
+                   const float* const* U, int R, float* T, float* P) {
+  const int64_t A = prod_range(shape, 0, N - 2), C = shape[N - 2] * shape[N - 1];
+  // T is the mode-0 MTTKRP of X seen as (A, I_{N-2}, I_{N-1}), P the last
+  // mode's of X seen as (I_0, .., I_{N-3}, C)
+  const int64_t tshape[3] = {A, shape[N - 2], shape[N - 1]};
+  const float* tf[3] = {nullptr, U[N - 2], U[N - 1]};
+  int64_t pshape[kMaxModes];
+  const float* pf[kMaxModes];
+  for (int m = 0; m < N - 2; ++m) {
+    pshape[m] = shape[m];
+    pf[m] = U[m];
+  }
+  pshape[N - 2] = C;
+  pf[N - 2] = nullptr;
+  for (int v = 0; v < 2; ++v) {
+    const int nd = v == 0 ? 3 : N - 1, mode = v == 0 ? 0 : N - 2;
+    const int64_t* sh = v == 0 ? tshape : pshape;
+    const int64_t rows = v == 0 ? A : C;
+    const ViewPlan plan = plan_view(ctx, nd, sh, mode, R, 0);
+    float* dst = v == 0 ? T : P;
+    float* out = dst;
+    if (plan.splits > 1) {
+      void* p;
+      TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(float) * (size_t)plan.splits * rows * R, &p));
+      out = (float*)p;
+    }
+    TSR_TRY(launch_view(ctx, ctx->stream, dX, nd, sh, mode, v == 0 ? tf : pf, R, plan, out));
+    if (plan.splits > 1)
+      TSR_TRY(launch_mttkrp_reduce(ctx, out, plan.splits, rows * R, dst));
+  }
+  return TSR_OK;
+}
+
 // Shared validation of tenrso's cp_reconstruct (outer.rs:231-255).
 int validate_reconstruct(int n_factors, const int64_t* fcols, int64_t n_weights, bool has_w) {
   if (n_factors <= 0)
@@ -820,28 +853,6 @@ int tsr_dense_create_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim, cons
   if (precision == TSR_PREC_FP32 && ndim >= 3 && vshape[0] <= ((int64_t)1 << 30) &&
       vshape[1] * vshape[2] < INT32_MAX) {
     const int64_t v2[2] = {vshape[0], vshape[1] * vshape[2]};
-    for (int m = 0; m < 2; ++m) {
-      // operand m: the 2-way view's mode-m unfolding (X, or its transpose)
-      size_t ab, bb;
-      mode_operand_bytes(make_unfolding(2, v2, m), precision, &ab, &bb);
-      void* buf = nullptr;
-      if (ab) {
-        if (cudaMalloc(&buf, ab) != cudaSuccess)
-          return cleanup(fail(TSR_E_CUDA, "cudaMalloc of %zu bytes failed", ab));
-        d->owned[2 * kMaxModes + 2 + m] = buf;
-      }
-      int rc = prepare_mode_into(ctx, d_tensor, 2, v2, m, precision, buf, nullptr, &d->vops[m]);
-      if (rc != TSR_OK) return cleanup(rc);
-    }
-    // the same bytes read as mode-0 unfoldings of finer tensors (their row
-    // strides equal the 2-way view's: round_up(cols, 8)), so that the FP32
-    // kernel forms the Khatri-Rao rows from the factors and may take its
-    // run-scaled form over the fastest other mode
-    d->vops[0].u = make_unfolding(3, vshape, 0);
-    int64_t tshape[kMaxModes];
-    tshape[0] = v2[1];
-    for (int p = 0; p < ndim - 2; ++p) tshape[1 + p] = shape[p];
-    d->vops[1].u = make_unfolding(ndim - 1, tshape, 0);
     d->v2_on = true;
     d->v2_shape[0] = v2[0];
     d->v2_shape[1] = v2[1];
@@ -1035,34 +1046,15 @@ int tsr_cp_loss_grad_dev_f32(tsr_ctx* ctx, const tsr_dense* X, const float* cons
     return contract_grad(ts.T, ts.P);
   }
   if (X->v2_on && R <= 32) {
-    // FP32: T is the mode-0 MTTKRP of X as (A, I_{N-2}, I_{N-1}), P that of
-    // X's transpose as (C, I_0, .., I_{N-3}): two passes over X's bytes
-    // instead of one per mode, and half the FLOPs of N MTTKRPs
+    // FP32: T = X KR(trailing two) and P = X^T KR(leading), both read from X
+    // in place: two passes over X's bytes instead of one per mode, and half
+    // the FLOPs of N MTTKRPs
     const int64_t A = X->v2_shape[0], C = X->v2_shape[1];
     void* tp;
     TSR_TRY(slot_get(ctx, SLOT_MISC0, sizeof(float) * (A + C) * R, &tp));
-    FactorTable f0{}, f1{};
-    f0.ptr[0] = d_factors[0];  // the output mode's slot (not read)
-    f0.rows[0] = A;
-    f0.ptr[1] = d_factors[N - 2];
-    f0.rows[1] = X->shape[N - 2];
-    f0.ptr[2] = d_factors[N - 1];
-    f0.rows[2] = X->shape[N - 1];
-    f1.ptr[0] = d_factors[0];  // not read
-    f1.rows[0] = C;
-    for (int p = 0; p < N - 2; ++p) {
-      f1.ptr[1 + p] = d_factors[p];
-      f1.rows[1 + p] = X->shape[p];
-    }
     float* T = (float*)tp;
     float* P = T + A * R;
-    for (int v = 0; v < 2; ++v) {
-      float* partials;
-      int splits;
-      TSR_TRY(run_mttkrp_partials(ctx, X->vops[v], v == 0 ? f0 : f1, R, TSR_PREC_FP32,
-                                  &partials, &splits));
-      TSR_TRY(launch_mttkrp_reduce(ctx, partials, splits, (v == 0 ? A : C) * R, v == 0 ? T : P));
-    }
+    TSR_TRY(contract_sides(ctx, X->dX, N, X->shape, d_factors, R, T, P));
     return contract_grad(T, P);
   }
   if (X->d3_on && X->d3_three && R <= 64) {

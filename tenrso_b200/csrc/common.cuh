@@ -211,18 +211,15 @@ struct Unfolding {
 };
 Unfolding make_unfolding(int ndim, const int64_t* shape, int mode);
 
-// Launch the (fp32) unfold of a row-major dense tensor into X_(mode) with row
-// stride u.ld. Pads columns [cols, ld) with zeros.
-int launch_unfold_f32(tsr_ctx* ctx, const float* X, const int64_t* shape, const Unfolding& u,
-                      float* out);
+// Unfold a row-major dense tensor into X_(mode) as bf16 hi / lo halves with
+// row stride u.ld. Pads columns [cols, ld) with zeros.
 int launch_unfold_bf16x2(tsr_ctx* ctx, const float* X, const int64_t* shape, const Unfolding& u,
                          __nv_bfloat16* hi, __nv_bfloat16* lo);
-// Every unfolding of a 3-way tensor in one pass (bf16 hi/lo for all modes, or
-// fp32 for modes 1 and 2), adding ||X||^2 into *norm_sq. Needs J, K multiples
-// of 8 (unpadded rows) and I <= 65535.
+// Every unfolding of a 3-way tensor in one pass (bf16 hi/lo), adding ||X||^2
+// into *norm_sq. Needs J, K multiples of 8 (unpadded rows) and I <= 65535.
 bool unfold3_supported(int ndim, const int64_t* shape);
-int launch_unfold3(tsr_ctx* ctx, const float* X, const int64_t* shape, bool bf16,
-                   void* const* hi, void* const* lo, double* norm_sq);
+int launch_unfold3(tsr_ctx* ctx, const float* X, const int64_t* shape, void* const* hi,
+                   void* const* lo, double* norm_sq);
 
 // Raise the dynamic shared-memory limits of every kernel once per process
 // (before any stream capture).

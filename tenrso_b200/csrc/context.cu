@@ -205,11 +205,6 @@ __global__ void unfold_transpose_kernel(const float* __restrict__ X, int64_t A, 
   }
 }
 
-struct StoreF32 {
-  float* out;
-  __device__ void operator()(int64_t k, float v) const { out[k] = v; }
-  __device__ void put4(int64_t k, float4 v) const { *reinterpret_cast<float4*>(out + k) = v; }
-};
 // x = hi + lo with hi = bf16(x), lo = bf16(x - hi): the operand split of the
 // BF16x3 MTTKRP.
 struct StoreBF16x2 {
@@ -238,38 +233,29 @@ struct StoreBF16x2 {
 // All unfoldings of a 3-way tensor X[I][J][K] (J, K multiples of 8; rows
 // unpadded) in one pass, plus ||X||^2:
 //   X_(0)[i][j*K + k], X_(1)[j][i*K + k], X_(2)[k][i*J + j]
-// as bf16 hi/lo pairs (BF16) or fp32 (modes 1 and 2 only: X is X_(0)). A CTA
-// owns a 32 (j) x 64 (k) tile of one slice i: it reads the tile once (128-bit
+// as bf16 hi/lo pairs. A CTA owns a 32 (j) x 64 (k) tile of one slice i: it reads the tile once (128-bit
 // loads), writes modes 0 and 1 as 16-byte row pieces and mode 2 through a
 // shared-memory transpose, 8 consecutive j per thread. Each element's split is
 // formed once for all three copies.
 struct Unfold3Out {
-  void* hi[3];  // bf16 hi (BF16) or fp32 (else); hi[0] unused for fp32
-  void* lo[3];  // bf16 lo (BF16 only)
+  __nv_bfloat16* hi[3];
+  __nv_bfloat16* lo[3];
 };
 
-template <bool BF16>
 __device__ __forceinline__ void put8(const Unfold3Out& o, int m, int64_t off, const float (&v)[8]) {
-  if (BF16) {
-    uint32_t h[4], l[4];
+  uint32_t h[4], l[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const __nv_bfloat162 hb = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-      const float2 hf = __bfloat1622float2(hb);
-      const __nv_bfloat162 lb = __floats2bfloat162_rn(v[2 * e] - hf.x, v[2 * e + 1] - hf.y);
-      h[e] = *reinterpret_cast<const uint32_t*>(&hb);
-      l[e] = *reinterpret_cast<const uint32_t*>(&lb);
-    }
-    *reinterpret_cast<uint4*>((__nv_bfloat16*)o.hi[m] + off) = make_uint4(h[0], h[1], h[2], h[3]);
-    *reinterpret_cast<uint4*>((__nv_bfloat16*)o.lo[m] + off) = make_uint4(l[0], l[1], l[2], l[3]);
-  } else {
-    float4* d = reinterpret_cast<float4*>((float*)o.hi[m] + off);
-    d[0] = make_float4(v[0], v[1], v[2], v[3]);
-    d[1] = make_float4(v[4], v[5], v[6], v[7]);
+  for (int e = 0; e < 4; ++e) {
+    const __nv_bfloat162 hb = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    const float2 hf = __bfloat1622float2(hb);
+    const __nv_bfloat162 lb = __floats2bfloat162_rn(v[2 * e] - hf.x, v[2 * e + 1] - hf.y);
+    h[e] = *reinterpret_cast<const uint32_t*>(&hb);
+    l[e] = *reinterpret_cast<const uint32_t*>(&lb);
   }
+  *reinterpret_cast<uint4*>(o.hi[m] + off) = make_uint4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<uint4*>(o.lo[m] + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-template <bool BF16>
 __global__ void __launch_bounds__(256) unfold3_kernel(const float* __restrict__ X, int I, int J,
                                                       int K, Unfold3Out o, double* norm_sq) {
   __shared__ float tile[64][33];  // [k][j]
@@ -288,8 +274,8 @@ __global__ void __launch_bounds__(256) unfold3_kernel(const float* __restrict__ 
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 #pragma unroll
     for (int e = 0; e < 8; ++e) ss += (double)v[e] * v[e];
-    if (BF16) put8<BF16>(o, 0, ((int64_t)i * J + j) * K + k0 + kl, v);
-    put8<BF16>(o, 1, ((int64_t)j * I + i) * K + k0 + kl, v);
+    put8(o, 0, ((int64_t)i * J + j) * K + k0 + kl, v);
+    put8(o, 1, ((int64_t)j * I + i) * K + k0 + kl, v);
   }
 #pragma unroll
   for (int e = 0; e < 8; ++e) tile[kl + e][jl] = in ? v[e] : 0.f;
@@ -299,7 +285,7 @@ __global__ void __launch_bounds__(256) unfold3_kernel(const float* __restrict__ 
     float w[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) w[e] = tile[kk][jq + e];
-    put8<BF16>(o, 2, ((int64_t)(k0 + kk) * I + i) * J + j0 + jq, w);
+    put8(o, 2, ((int64_t)(k0 + kk) * I + i) * J + j0 + jq, w);
   }
   for (int s = 16; s > 0; s >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, s);
   if ((t & 31) == 0) ws[t >> 5] = ss;
@@ -316,20 +302,17 @@ bool unfold3_supported(int ndim, const int64_t* shape) {
          shape[1] < (1 << 30) && shape[2] / 64 < 65535 && shape[0] * shape[1] * shape[2] > 0;
 }
 
-int launch_unfold3(tsr_ctx* ctx, const float* X, const int64_t* shape, bool bf16,
-                   void* const* hi, void* const* lo, double* norm_sq) {
+int launch_unfold3(tsr_ctx* ctx, const float* X, const int64_t* shape, void* const* hi,
+                   void* const* lo, double* norm_sq) {
   if (!unfold3_supported(3, shape)) return fail(TSR_E_UNSUPPORTED, "unfold3: shape");
   Unfold3Out o{};
   for (int m = 0; m < 3; ++m) {
-    o.hi[m] = hi[m];
-    o.lo[m] = lo ? lo[m] : nullptr;
+    o.hi[m] = (__nv_bfloat16*)hi[m];
+    o.lo[m] = (__nv_bfloat16*)lo[m];
   }
   const int I = (int)shape[0], J = (int)shape[1], K = (int)shape[2];
   dim3 grid((unsigned)ceil_div(J, 32), (unsigned)I, (unsigned)ceil_div(K, 64));
-  if (bf16)
-    unfold3_kernel<true><<<grid, 256, 0, ctx->stream>>>(X, I, J, K, o, norm_sq);
-  else
-    unfold3_kernel<false><<<grid, 256, 0, ctx->stream>>>(X, I, J, K, o, norm_sq);
+  unfold3_kernel<<<grid, 256, 0, ctx->stream>>>(X, I, J, K, o, norm_sq);
   ctx->launches++;
   TSR_CUDA(cudaGetLastError());
   return TSR_OK;
@@ -353,13 +336,6 @@ static int launch_unfold(tsr_ctx* ctx, const float* X, const int64_t* shape, con
   ctx->launches++;
   TSR_CUDA(cudaGetLastError());
   return TSR_OK;
-}
-
-int launch_unfold_f32(tsr_ctx* ctx, const float* X, const int64_t* shape, const Unfolding& u,
-                      float* out) {
-  if (u.ld != u.cols)
-    TSR_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * u.rows * u.ld, ctx->stream));
-  return launch_unfold(ctx, X, shape, u, StoreF32{out});
 }
 
 int launch_unfold_bf16x2(tsr_ctx* ctx, const float* X, const int64_t* shape, const Unfolding& u,

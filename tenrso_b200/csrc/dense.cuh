@@ -2,7 +2,7 @@
 // adjoint: argument validation in tenrso's wording, host staging, per-mode
 // MTTKRP operands and the split-K MTTKRP launch.
 #pragma once
-#include "mttkrp.cuh"
+#include "view.cuh"
 
 namespace tsr {
 
@@ -21,11 +21,12 @@ int upload_tensor(tsr_ctx* ctx, const float* host, int ndim, const int64_t* shap
 int upload_factors(tsr_ctx* ctx, int ndim, const int64_t* shape, const float* const* factors,
                    int64_t R, FactorTable* ft);
 
-// Per-mode operand of the MTTKRP: the mode's unfolding in the precision the
-// kernel reads (fp32, or the bf16 hi/lo halves).
+// Per-mode operand of the MTTKRP. FP32: the tensor itself, read in place.
+// BF16x3: the mode's unfolding as bf16 hi / lo halves.
 struct ModeOperand {
   Unfolding u;
   const float* f32 = nullptr;
+  int64_t shape[kMaxModes] = {};
   const __nv_bfloat16* hi = nullptr;
   const __nv_bfloat16* lo = nullptr;
   // written before any kernel that precedes the MTTKRP in its stream (e.g.
@@ -41,8 +42,8 @@ int prepare_mode_into(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* sh
 // Same, with buffers from the context's unfolding slots (slot_index 0..7).
 int prepare_mode(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape, int mode,
                  int precision, int slot_index, ModeOperand* op);
-// Run length of an FP32 operand for the run-scaled SIMT kernel (0: not usable).
-int64_t simt_run_len(const ModeOperand& op);
+// Partial floats run_mttkrp_partials will need for this operand.
+size_t mode_partial_floats(const tsr_ctx* ctx, const ModeOperand& op, int R, int precision);
 // Split-K partial MTTKRP of one mode into the context's partial slot.
 int run_mttkrp_partials(tsr_ctx* ctx, const ModeOperand& op, const FactorTable& ft, int R,
                         int precision, float** partials, int* splits);

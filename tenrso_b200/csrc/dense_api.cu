@@ -133,14 +133,9 @@ void seeded_uniform(uint64_t seed, uint64_t stream, int64_t n, float* out) {
   }
 }
 
-// Per-mode operand of the MTTKRP: unfolding copies in the precision needed.
+// Per-mode operand of the MTTKRP: bf16 unfolding copies, or the tensor itself.
 void mode_operand_bytes(const Unfolding& u, int precision, size_t* a_bytes, size_t* b_bytes) {
-  if (precision == TSR_PREC_BF16X3) {
-    *a_bytes = *b_bytes = 2 * (size_t)u.rows * u.ld;
-  } else {
-    *a_bytes = (u.mode == 0 && u.ld == u.cols) ? 0 : sizeof(float) * (size_t)u.rows * u.ld;
-    *b_bytes = 0;
-  }
+  *a_bytes = *b_bytes = precision == TSR_PREC_BF16X3 ? 2 * (size_t)u.rows * u.ld : 0;
 }
 
 int prepare_mode_into(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape, int mode,
@@ -154,13 +149,8 @@ int prepare_mode_into(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* sh
     op->lo = (const __nv_bfloat16*)buf_b;
     return TSR_OK;
   }
-  // mode 0 of a row-major tensor is already its unfolding when rows are aligned
-  if (mode == 0 && u.ld == u.cols) {
-    op->f32 = dX;
-    return TSR_OK;
-  }
-  TSR_TRY(launch_unfold_f32(ctx, dX, shape, u, (float*)buf_a));
-  op->f32 = (const float*)buf_a;
+  op->f32 = dX;
+  for (int m = 0; m < ndim; ++m) op->shape[m] = shape[m];
   return TSR_OK;
 }
 
@@ -174,32 +164,38 @@ int prepare_mode(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape, 
   return prepare_mode_into(ctx, dX, ndim, shape, mode, precision, a, b, op);
 }
 
-// Split-K partial MTTKRP of one mode into `partials` (allocated here).
-// Run length of the FP32 operand for the run-scaled kernel (the fastest other
-// mode), or 0 when its rows are not 16-byte aligned.
-int64_t simt_run_len(const ModeOperand& op) {
-  if (!op.f32 || ((uintptr_t)op.f32 & 15) != 0 || (op.u.ld & 3) != 0 || op.u.n_other < 1)
-    return 0;
-  return op.u.other_size[op.u.n_other - 1];
+// A captured sweep leaves some SMs to the FP64 kernels beside it.
+static ViewPlan plan_mode_view(const tsr_ctx* ctx, const ModeOperand& op, int R) {
+  return plan_view(ctx, op.u.ndim, op.shape, op.u.mode, R, op.resident ? ctx->reserve_sms : 0);
 }
 
+size_t mode_partial_floats(const tsr_ctx* ctx, const ModeOperand& op, int R, int precision) {
+  const int64_t splits = precision == TSR_PREC_BF16X3 ? plan_tc(ctx, op.u, R).splits
+                                                      : plan_mode_view(ctx, op, R).splits;
+  return (size_t)splits * op.u.rows * R;
+}
+
+// Split-K partial MTTKRP of one mode into `partials` (allocated here).
 int run_mttkrp_partials(tsr_ctx* ctx, const ModeOperand& op, const FactorTable& ft, int R,
                         int precision, float** partials, int* splits) {
-  KRSpec kr = make_krspec(op.u, ft, R);
-  SplitPlan plan;
-  bool tc = precision == TSR_PREC_BF16X3;
-  if (tc && !tc_supported(op.u, R))
-    return fail(TSR_E_UNSUPPORTED, "BF16X3 path needs rank <= 256 (got %d)", R);
-  plan = tc ? plan_tc(ctx, op.u, R)
-            : plan_simt(ctx, op.u.rows, op.u.cols, R, simt_run_len(op));
   void* p;
-  TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(float) * partial_floats(plan, op.u.rows, R), &p));
-  if (tc)
-    TSR_TRY(launch_mttkrp_tc(ctx, op.hi, op.lo, op.u, kr, plan, (float*)p, op.resident));
-  else
-    TSR_TRY(launch_mttkrp_simt(ctx, op.f32, op.u, kr, plan, (float*)p));
+  if (precision == TSR_PREC_BF16X3) {
+    if (!tc_supported(op.u, R))
+      return fail(TSR_E_UNSUPPORTED, "BF16X3 path needs rank <= 256 (got %d)", R);
+    const SplitPlan plan = plan_tc(ctx, op.u, R);
+    TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(float) * partial_floats(plan, op.u.rows, R), &p));
+    TSR_TRY(launch_mttkrp_tc(ctx, op.hi, op.lo, op.u, make_krspec(op.u, ft, R), plan, (float*)p,
+                             op.resident));
+    *splits = plan.splits;
+  } else {
+    const ViewPlan plan = plan_mode_view(ctx, op, R);
+    TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(float) * (size_t)plan.splits * op.u.rows * R,
+                     &p));
+    TSR_TRY(launch_view(ctx, ctx->stream, op.f32, op.u.ndim, op.shape, op.u.mode, ft.ptr, R,
+                        plan, (float*)p));
+    *splits = plan.splits;
+  }
   *partials = (float*)p;
-  *splits = plan.splits;
   return TSR_OK;
 }
 
@@ -456,7 +452,8 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
   const bool d3 = !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
                   dense3_supported(ndim, shape, R) && ((uintptr_t)dX & 15) == 0 &&
                   !(cons && cons->orthogonal);
-  const bool fused_unfold = !d3 && !sp && max_iters > 0 && unfold3_supported(ndim, shape);
+  const bool fused_unfold = !d3 && !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
+                            unfold3_supported(ndim, shape);
   if (d3) {
     Dense3& d = a.d3;
     a.d3_on = 1;
@@ -514,20 +511,13 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
         mode_operand_bytes(ops[m].u, precision, &ab, &bb);
         if (ab) TSR_TRY(slot_get(ctx, SLOT_UNFOLD0 + m, ab, &uhi[m]));
         if (bb) TSR_TRY(slot_get(ctx, SLOT_UNFOLD_LO + m, bb, &ulo[m]));
-        if (precision == TSR_PREC_BF16X3) {
-          ops[m].hi = (const __nv_bfloat16*)uhi[m];
-          ops[m].lo = (const __nv_bfloat16*)ulo[m];
-        } else {
-          ops[m].f32 = m == 0 ? dX : (const float*)uhi[m];
-        }
+        ops[m].hi = (const __nv_bfloat16*)uhi[m];
+        ops[m].lo = (const __nv_bfloat16*)ulo[m];
       } else {
         TSR_TRY(prepare_mode(ctx, dX, ndim, shape, m, precision, m, &ops[m]));
       }
-      const bool tc = precision == TSR_PREC_BF16X3;
-      SplitPlan p = tc ? plan_tc(ctx, ops[m].u, R)
-                       : plan_simt(ctx, ops[m].u.rows, ops[m].u.cols, R, simt_run_len(ops[m]));
-      pmax = std::max(pmax, partial_floats(p, ops[m].u.rows, R));
       ops[m].resident = true;  // prepared here, before the sweep is enqueued
+      pmax = std::max(pmax, mode_partial_floats(ctx, ops[m], R, precision));
       a.op_ptrs[3 * m] = ops[m].f32;
       a.op_ptrs[3 * m + 1] = ops[m].hi;
       a.op_ptrs[3 * m + 2] = ops[m].lo;
@@ -535,29 +525,29 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
     void* pp;
     TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(float) * pmax, &pp));
     a.partials = (float*)pp;
-    if (fused_unfold) {
-      // the initial Grams run on the aux stream beside the unfold pass
-      TSR_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
-      TSR_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
-      for (int m = 0; m < ndim; ++m)
-        TSR_TRY(launch_gram(ctx, ctx->aux, a.ft.ptr[m], shape[m], R,
-                            a.b.grams + (size_t)m * R * R, false));
-      TSR_CUDA(cudaEventRecord(ctx->ev[1], ctx->aux));
-      TSR_TRY(launch_unfold3(ctx, dX, shape, precision == TSR_PREC_BF16X3, uhi,
-                             precision == TSR_PREC_BF16X3 ? ulo : nullptr,
-                             &a.b.state->xnorm_sq));
-      TSR_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev[1], 0));
-    }
+    // the initial Grams run on the aux stream beside the pass that forms
+    // ||X||^2 (with the unfoldings, where the fused unfold applies)
+    TSR_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
+    TSR_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
+    for (int m = 0; m < ndim; ++m)
+      TSR_TRY(launch_gram(ctx, ctx->aux, a.ft.ptr[m], shape[m], R,
+                          a.b.grams + (size_t)m * R * R, false));
+    TSR_CUDA(cudaEventRecord(ctx->ev[1], ctx->aux));
+    if (fused_unfold)
+      TSR_TRY(launch_unfold3(ctx, dX, shape, uhi, ulo, &a.b.state->xnorm_sq));
+    else
+      TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
+    TSR_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev[1], 0));
   }
   if (sp)  // sum of squared values, FP64, computed when the tensor was built
     TSR_CUDA(cudaMemcpyAsync(&a.b.state->xnorm_sq, &sp->norm_sq, sizeof(double),
                              cudaMemcpyHostToDevice, ctx->stream));
-  else if (!fused_unfold && !d3)
-    TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
-  if (!fused_unfold && !d3)
+  if (sp || max_iters <= 0) {
+    if (!sp) TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
     for (int m = 0; m < ndim; ++m)
       TSR_TRY(launch_gram(ctx, ctx->stream, a.ft.ptr[m], shape[m], R,
                           a.b.grams + (size_t)m * R * R, false));
+  }
 
   const bool time_limited = time_limit_s >= 0.0;
   bool stopped_by_time = false;
@@ -690,6 +680,7 @@ void init_kernel_attributes() {
   init_tc_attributes();
   init_mttkrp3_attributes();
   init_simt_attributes();
+  init_view_attributes();
   init_als_attributes();
   init_adjoint_attributes();
   init_csf_attributes();

@@ -1,0 +1,165 @@
+// Planning and launch of the view kernels (see view.cuh): the FP32 MTTKRP of
+// every dense entry point.
+#include "view.cuh"
+
+#include <algorithm>
+#include <cstring>
+
+namespace tsr {
+
+namespace {
+
+constexpr int kWidths[] = {16, 24, 32, 48, 64};
+constexpr int kRows[] = {32, 48, 64, 96, 128};
+constexpr int64_t VIEW_MIN_RUN = 16;
+int g_ctas[5][5];  // resident CTAs per SM, filled by init_view_attributes
+
+int width_index(int bn) {
+  for (int i = 0; i < 5; ++i)
+    if (kWidths[i] == bn) return i;
+  return 4;
+}
+int rows_index(int bm) {
+  for (int i = 0; i < 5; ++i)
+    if (kRows[i] == bm) return i;
+  return 4;
+}
+
+int dispatch(tsr_ctx* ctx, cudaStream_t s, const ViewArgs& g, int bn, int bm, dim3 grid) {
+  switch (bn) {
+    case 16: return launch_view_bn<16>(ctx, s, g, bm, grid);
+    case 24: return launch_view_bn<24>(ctx, s, g, bm, grid);
+    case 32: return launch_view_bn<32>(ctx, s, g, bm, grid);
+    case 48: return launch_view_bn<48>(ctx, s, g, bm, grid);
+    default: return launch_view_bn<64>(ctx, s, g, bm, grid);
+  }
+}
+
+// The narrowest tile that holds R (or an equal share of R beyond 64), and the
+// tile height with the least padded work: a tile of m rows costs about m + 16
+// (its FMAs, and the share of K's tile and of the barriers).
+void choose_tile(int64_t rows, int R, int* bn, int* bm) {
+  const int64_t nt = ceil_div(R, 64), share = ceil_div(R, nt);
+  *bn = 64;
+  for (int w : kWidths)
+    if (w >= share) {
+      *bn = w;
+      break;
+    }
+  int64_t best = INT64_MAX;
+  for (int i = 4; i >= 0; --i) {
+    const int64_t cost = ceil_div(rows, kRows[i]) * (kRows[i] + 16);
+    if (cost < best) {
+      best = cost;
+      *bm = kRows[i];
+    }
+  }
+}
+
+// The contraction of one mode: which contracted mode is the inner one and the
+// strides of all of them. The inner mode is the fastest contracted one, where
+// a chunk is contiguous in memory (or, for the last mode's MTTKRP, its rows
+// are); one shorter than half a chunk would leave most of each step empty, so
+// then it is the longest one.
+void describe(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner) {
+  int64_t stride[kMaxModes], st = 1;
+  for (int m = ndim - 1; m >= 0; --m) {
+    stride[m] = st;
+    st *= shape[m];
+  }
+  int in = mode == ndim - 1 ? ndim - 2 : ndim - 1;
+  if (shape[in] < VIEW_MIN_RUN)
+    for (int m = ndim - 1; m >= 0; --m)
+      if (m != mode && shape[m] > shape[in]) in = m;
+  *inner = in;
+  g->rows = shape[mode];
+  g->row_stride = stride[mode];
+  g->k_stride = stride[in];
+  g->S = (uint32_t)shape[in];
+  int64_t runs = 1;
+  for (int m = 0; m < ndim; ++m) {
+    if (m == mode || m == in) continue;
+    g->size[g->n_outer] = (uint32_t)shape[m];
+    g->stride[g->n_outer] = stride[m];
+    ++g->n_outer;
+    runs *= shape[m];
+  }
+  // equal chunks of at most 32 columns
+  g->chunks = (uint32_t)ceil_div(g->S, 32);
+  g->kc = (int)round_up(ceil_div(g->S, g->chunks), 4);
+  g->chunks = (uint32_t)ceil_div(g->S, g->kc);
+  g->steps = runs * g->chunks;
+}
+
+int tile_map(const ViewArgs& g) {
+  if (g.k_stride != 1) return VIEW_ACROSS;
+  bool vec = ((uintptr_t)g.X & 15) == 0 && g.S % 4 == 0 && g.row_stride % 4 == 0 &&
+             g.x_batch % 4 == 0;
+  for (int p = 0; p < g.n_outer; ++p) vec = vec && g.stride[p] % 4 == 0;
+  return vec ? VIEW_VEC : VIEW_ALONG;
+}
+
+}  // namespace
+
+void init_view_attributes() {
+  for (int i = 0; i < 5; ++i) {
+    g_ctas[0][i] = view_ctas_per_sm<16>(kRows[i]);
+    g_ctas[1][i] = view_ctas_per_sm<24>(kRows[i]);
+    g_ctas[2][i] = view_ctas_per_sm<32>(kRows[i]);
+    g_ctas[3][i] = view_ctas_per_sm<48>(kRows[i]);
+    g_ctas[4][i] = view_ctas_per_sm<64>(kRows[i]);
+  }
+}
+
+ViewPlan plan_view(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
+                   int reserve) {
+  ViewPlan p;
+  ViewArgs g;
+  std::memset(&g, 0, sizeof(g));
+  int inner;
+  choose_tile(shape[mode], R, &p.bn, &p.bm);
+  describe(ndim, shape, mode, &g, &inner);
+  const int per_sm = std::max(1, g_ctas[width_index(p.bn)][rows_index(p.bm)]);
+  const int64_t tiles = ceil_div(g.rows, p.bm) * ceil_div(R, p.bn);
+  const int64_t slots = (int64_t)std::max(1, ctx->sm_count - reserve) * per_sm;
+  // one wave of resident CTAs, but no more splits than SMs where a split would
+  // be left with fewer than four steps
+  const int64_t few = std::max<int64_t>(ceil_div(g.steps, 4), ctx->sm_count - reserve);
+  const int64_t want = std::max<int64_t>(
+      1, std::min<int64_t>({slots / tiles, std::min(few, g.steps), (int64_t)65535}));
+  p.steps_per_split = ceil_div(g.steps, want);
+  p.splits = (int)ceil_div(g.steps, p.steps_per_split);
+  return p;
+}
+
+int launch_view(tsr_ctx* ctx, cudaStream_t s, const float* X, int ndim, const int64_t* shape,
+                int mode, const float* const* f, int R, const ViewPlan& plan, float* partials) {
+  ViewArgs g;
+  std::memset(&g, 0, sizeof(g));
+  int inner;
+  describe(ndim, shape, mode, &g, &inner);
+  int64_t cols = 1;
+  for (int m = 0; m < ndim; ++m)
+    if (m != mode) cols *= shape[m];
+  if (cols >= (int64_t)UINT32_MAX) return fail(TSR_E_UNSUPPORTED, "unfolding too wide");
+  g.X = X;
+  g.steps_per_split = plan.steps_per_split;
+  g.R = R;
+  g.inner = f[inner];
+  g.inner_s = R;
+  g.inner_c = 1;
+  g.inner_vec = R % 4 == 0 && ((uintptr_t)f[inner] & 15) == 0;
+  for (int m = 0, p = 0; m < ndim; ++m)
+    if (m != mode && m != inner) g.f[p++] = f[m];
+  g.out = partials;
+  g.out_split = g.rows * R;
+  g.out_row = R;
+  g.out_col = 1;
+  g.map = tile_map(g);
+  dim3 grid((unsigned)ceil_div(g.rows, plan.bm), (unsigned)plan.splits,
+            (unsigned)ceil_div(R, plan.bn));
+  if (grid.z > 65535) return fail(TSR_E_UNSUPPORTED, "MTTKRP grid too large");
+  return dispatch(ctx, s, g, plan.bn, plan.bm, grid);
+}
+
+}  // namespace tsr
