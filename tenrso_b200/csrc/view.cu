@@ -92,7 +92,7 @@ void describe(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner)
 }
 
 int tile_map(const ViewArgs& g) {
-  if (g.k_stride != 1) return VIEW_ACROSS;
+  if (g.k_stride != 1) return g.row_stride == 1 ? VIEW_ACROSS : VIEW_STRIDED;
   bool vec = ((uintptr_t)g.X & 15) == 0 && g.S % 4 == 0 && g.row_stride % 4 == 0 &&
              g.x_batch % 4 == 0;
   for (int p = 0; p < g.n_outer; ++p) vec = vec && g.stride[p] % 4 == 0;

@@ -46,8 +46,9 @@ struct ViewArgs {
 
 // Tile load patterns: VEC reads 16 bytes along a run (everything a multiple of
 // 4 floats), ALONG one float per lane along a run, ACROSS 8 rows x 4 columns
-// per warp (the row index is the tensor's contiguous direction).
-enum ViewMap { VIEW_VEC = 0, VIEW_ALONG = 1, VIEW_ACROSS = 2 };
+// per warp (the row index is the tensor's contiguous direction), STRIDED the
+// same where neither direction is contiguous.
+enum ViewMap { VIEW_VEC = 0, VIEW_ALONG = 1, VIEW_ACROSS = 2, VIEW_STRIDED = 3 };
 
 struct ViewPlan {
   int bn = 32;  // output columns per CTA

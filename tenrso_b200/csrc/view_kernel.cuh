@@ -150,11 +150,22 @@ view_kernel(const __grid_constant__ ViewArgs g) {
       } else if (MAP == VIEW_ALONG) {  // 32 columns of a row
         if (lane < g.kc)
           column(dst + lane, run + s0 + lane + w * g.row_stride, w, ViewInt<NW>(), lane < valid);
-      } else {  // 4 columns of 8 rows
-        const int m = w * 8 + (lane & 7);
-        const float* src = run + m * g.row_stride;
-        for (int k = lane >> 3; k < g.kc; k += 4)
-          column(dst + k, src + (s0 + k) * g.k_stride, m, ViewInt<NW * 8>(), k < valid);
+      } else {  // 4 columns of 8 rows; neighbouring rows (ACROSS) at constant offsets
+        constexpr int ST = NW * 8, IT = (BM + ST - 1) / ST;
+        const int64_t rs = MAP == VIEW_ACROSS ? 1 : g.row_stride;
+        const int m = w * 8 + (lane & 7), kl = lane >> 3;
+        const int n = m < rows_here ? (rows_here - m + ST - 1) / ST : 0;
+        const float* src = run + m * rs + (s0 + kl) * g.k_stride;
+        dst += m * VPITCH + kl;
+        for (int k = kl; k < g.kc; k += 4) {
+          const bool in = k < valid;
+          const float* sp = in ? src : g.X;
+#pragma unroll
+          for (int q = 0; q < IT; ++q)
+            if (q < n) view_cp4(dst + q * ST * VPITCH, sp + q * ST * rs, in);
+          src += 4 * g.k_stride;
+          dst += 4;
+        }
       }
       // K's rows: columns past R and rows past the run are zero (the X values
       // the latter meet are zero-filled too: nothing non-finite leaks in)
@@ -295,8 +306,9 @@ int view_occ() {
   constexpr size_t sm = view_smem<BN, RPT>();
   cudaFuncSetAttribute(view_kernel<BN, RPT, MAP, false>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  cudaFuncSetAttribute(view_kernel<BN, RPT, MAP, true>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if constexpr (MAP != VIEW_STRIDED)  // batched products have a contiguous side
+    cudaFuncSetAttribute(view_kernel<BN, RPT, MAP, true>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   int n = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, view_kernel<BN, RPT, MAP, false>,
                                                 4 * BN, sm);
@@ -304,10 +316,11 @@ int view_occ() {
 }
 template <int BN, int RPT>
 int view_occ_min() {
-  const int a = view_occ<BN, RPT, VIEW_VEC>(), b = view_occ<BN, RPT, VIEW_ALONG>(),
-            c = view_occ<BN, RPT, VIEW_ACROSS>();
-  const int ab = a < b ? a : b;
-  return ab < c ? ab : c;
+  const int n[4] = {view_occ<BN, RPT, VIEW_VEC>(), view_occ<BN, RPT, VIEW_ALONG>(),
+                    view_occ<BN, RPT, VIEW_ACROSS>(), view_occ<BN, RPT, VIEW_STRIDED>()};
+  int least = n[0];
+  for (int v : n) least = v < least ? v : least;
+  return least;
 }
 
 template <int BN, int RPT, bool BATCHED>
@@ -317,7 +330,10 @@ void view_map(cudaStream_t s, const ViewArgs& g, dim3 grid) {
   if (g.map == VIEW_VEC) view_kernel<BN, RPT, VIEW_VEC, BATCHED><<<grid, nt, sm, s>>>(g);
   else if (g.map == VIEW_ALONG)
     view_kernel<BN, RPT, VIEW_ALONG, BATCHED><<<grid, nt, sm, s>>>(g);
-  else view_kernel<BN, RPT, VIEW_ACROSS, BATCHED><<<grid, nt, sm, s>>>(g);
+  else if (g.map == VIEW_ACROSS)
+    view_kernel<BN, RPT, VIEW_ACROSS, BATCHED><<<grid, nt, sm, s>>>(g);
+  else if constexpr (!BATCHED)
+    view_kernel<BN, RPT, VIEW_STRIDED, false><<<grid, nt, sm, s>>>(g);
 }
 template <int BN, int RPT>
 void view_go(cudaStream_t s, const ViewArgs& g, dim3 grid) {
