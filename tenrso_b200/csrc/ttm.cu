@@ -12,101 +12,16 @@
 // GEMM C_a (J x B) = M (J x I) . X_a (I x B); for the last mode (B = 1) the
 // whole product is one GEMM Y (A x J) = X (A x I) . M^T.
 //
-// The kernel: 64 x 64 output tile per 256-thread CTA (4 x 4 per thread),
-// 16-deep K slices staged in shared memory, fp32 FMA with fp32 accumulation
-// (the reference's sum is in T), operands addressed by (row, column) strides
-// so that both layouts share it.
+// Both run the view kernels (view.cuh) with the matrix as the contraction's
+// second operand: X is read in place, one float per lane or 16 bytes along its
+// contiguous direction, and the products are fp32 FMAs summed in chains of 16
+// (the reference's sum is in T).
 #include <algorithm>
 #include <vector>
 
 #include "dense.cuh"
 
 namespace tsr {
-
-namespace {
-
-struct GemmView {
-  const float* a;  // op A (m x k): a[m * a_rs + k * a_cs]
-  int64_t a_rs, a_cs;
-  const float* b;  // op B (k x n): b[k * b_rs + n * b_cs] (+ batch * b_bs)
-  int64_t b_rs, b_cs, b_bs;
-  float* c;        // C (m x n): c[m * c_rs + n] (+ batch * c_bs)
-  int64_t c_rs, c_bs;
-  int64_t M, N, K;
-  int64_t batch;
-};
-
-constexpr int TT_BM = 64, TT_BN = 64, TT_BK = 16;
-
-__global__ void __launch_bounds__(256) ttm_gemm_kernel(GemmView g) {
-  __shared__ float As[TT_BK][TT_BM + 4];
-  __shared__ float Bs[TT_BK][TT_BN + 4];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t m0 = (int64_t)blockIdx.y * TT_BM, n0 = (int64_t)blockIdx.x * TT_BN;
-  for (int64_t z = blockIdx.z; z < g.batch; z += gridDim.z) {
-  const float* bz = g.b + z * g.b_bs;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  for (int64_t k0 = 0; k0 < g.K; k0 += TT_BK) {
-    // A tile (BM x BK) and B tile (BK x BN): 1024 elements each, 4 per
-    // thread; the thread index runs along the operand's contiguous side
-    for (int e = threadIdx.x; e < TT_BM * TT_BK; e += 256) {
-      int r, c;
-      if (g.a_cs == 1) {
-        r = e / TT_BK;
-        c = e % TT_BK;
-      } else {
-        r = e % TT_BM;
-        c = e / TT_BM;
-      }
-      const int64_t m = m0 + r, k = k0 + c;
-      As[c][r] = (m < g.M && k < g.K) ? __ldg(g.a + m * g.a_rs + k * g.a_cs) : 0.f;
-    }
-    for (int e = threadIdx.x; e < TT_BK * TT_BN; e += 256) {
-      int r, c;
-      if (g.b_cs == 1) {
-        r = e / TT_BN;
-        c = e % TT_BN;
-      } else {
-        r = e % TT_BK;
-        c = e / TT_BK;
-      }
-      const int64_t k = k0 + r, n = n0 + c;
-      Bs[r][c] = (k < g.K && n < g.N) ? __ldg(bz + k * g.b_rs + n * g.b_cs) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TT_BK; ++kk) {
-      float av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bv[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  float* cz = g.c + z * g.c_bs;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t m = m0 + ty + 16 * i;
-    if (m >= g.M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t n = n0 + tx + 16 * j;
-      if (n < g.N) cz[m * g.c_rs + n] = acc[i][j];
-    }
-  }
-  }
-}
-
-}  // namespace
 
 // Y = X x_mode M on device buffers (X: shape, row-major; M: J x shape[mode],
 // row-major; Y: shape with shape[mode] -> J).
@@ -117,49 +32,7 @@ int launch_ttm(tsr_ctx* ctx, cudaStream_t s, const float* X, int ndim, const int
   for (int m = mode + 1; m < ndim; ++m) B *= shape[m];
   const int64_t I = shape[mode];
   if (A * B * J == 0) return TSR_OK;
-  GemmView g;
-  int64_t batch;
-  if (B > 1) {
-    // C_a (J x B) = M (J x I) . X_a (I x B)
-    g.a = Mat;
-    g.a_rs = I;
-    g.a_cs = 1;
-    g.b = X;
-    g.b_rs = B;
-    g.b_cs = 1;
-    g.b_bs = I * B;
-    g.c = Y;
-    g.c_rs = B;
-    g.c_bs = J * B;
-    g.M = J;
-    g.N = B;
-    g.K = I;
-    batch = A;
-  } else {
-    // Y (A x J) = X (A x I) . M^T
-    g.a = X;
-    g.a_rs = I;
-    g.a_cs = 1;
-    g.b = Mat;
-    g.b_rs = 1;
-    g.b_cs = I;
-    g.b_bs = 0;
-    g.c = Y;
-    g.c_rs = J;
-    g.c_bs = 0;
-    g.M = A;
-    g.N = J;
-    g.K = I;
-    batch = 1;
-  }
-  g.batch = batch;
-  dim3 grid((unsigned)ceil_div(g.N, TT_BN), (unsigned)ceil_div(g.M, TT_BM),
-            (unsigned)std::min<int64_t>(batch, 65535));
-  if (grid.y > 65535u) return fail(TSR_E_UNSUPPORTED, "output too tall for one launch");
-  ttm_gemm_kernel<<<grid, 256, 0, s>>>(g);
-  ctx->launches++;
-  TSR_CUDA(cudaGetLastError());
-  return TSR_OK;
+  return launch_view_matrix(ctx, s, X, A, I, B, Mat, J, Y);
 }
 
 namespace {

@@ -56,6 +56,28 @@ void choose_tile(int64_t rows, int R, int* bn, int* bm) {
   }
 }
 
+// Tile of a product that is not split over its contraction: the least work of
+// the busiest SM (its tiles, each padded by the fixed part of a step), weighted
+// by how well the warps it holds cover latency (w / (w + 4): 8 warps reach two
+// thirds, 16 four fifths of the rate of a full SM).
+void choose_tile_unsplit(const tsr_ctx* ctx, int64_t rows, int64_t R, int64_t batch, int* bn,
+                         int* bm) {
+  double best = 0.0;
+  for (int wi = 0; wi < 5; ++wi)
+    for (int ri = 0; ri < 5; ++ri) {
+      const int w = kWidths[wi], m = kRows[ri];
+      const int64_t tiles = ceil_div(rows, m) * ceil_div(R, w) * batch;
+      const int64_t per_sm = ceil_div(tiles, ctx->sm_count);
+      const double warps = (double)std::min<int64_t>(g_ctas[wi][ri], per_sm) * (w / 8);
+      const double cost = (double)per_sm * (m + 16) * (w + 8) * (warps + 4) / warps;
+      if (best == 0.0 || cost < best) {
+        best = cost;
+        *bn = w;
+        *bm = m;
+      }
+    }
+}
+
 // The contraction of one mode: which contracted mode is the inner one and the
 // strides of all of them. The inner mode is the fastest contracted one, where
 // a chunk is contiguous in memory (or, for the last mode's MTTKRP, its rows
@@ -160,6 +182,57 @@ int launch_view(tsr_ctx* ctx, cudaStream_t s, const float* X, int ndim, const in
             (unsigned)ceil_div(R, plan.bn));
   if (grid.z > 65535) return fail(TSR_E_UNSUPPORTED, "MTTKRP grid too large");
   return dispatch(ctx, s, g, plan.bn, plan.bm, grid);
+}
+
+int launch_view_matrix(tsr_ctx* ctx, cudaStream_t s, const float* X, int64_t A, int64_t I,
+                       int64_t B, const float* mat, int64_t J, float* Y) {
+  if (ceil_div(B > 1 ? J : A, 64) > 65535)
+    return fail(TSR_E_UNSUPPORTED, "output too tall for one launch");
+  if (I > (int64_t)UINT32_MAX - 64) return fail(TSR_E_UNSUPPORTED, "contracted mode too long");
+  if (I == 0) {  // an empty sum
+    TSR_CUDA(cudaMemsetAsync(Y, 0, sizeof(float) * A * J * B, s));
+    return TSR_OK;
+  }
+  ViewArgs g;
+  std::memset(&g, 0, sizeof(g));
+  g.X = X;
+  g.S = (uint32_t)I;
+  g.chunks = (uint32_t)ceil_div(I, 32);
+  g.kc = (int)round_up(ceil_div(I, g.chunks), 4);
+  g.chunks = (uint32_t)ceil_div(I, g.kc);
+  g.steps = g.steps_per_split = g.chunks;
+  g.inner_s = 1;
+  g.inner_c = I;
+  if (B > 1) {  // per a: rows b, columns i at stride B; Y's contiguous direction is b
+    g.rows = B;
+    g.row_stride = 1;
+    g.k_stride = B;
+    g.out_row = 1;
+    g.out_col = B;
+    g.batch = A;
+    g.x_batch = I * B;
+    g.out_batch = J * B;
+  } else {  // the last mode: rows a of I columns
+    g.rows = A;
+    g.row_stride = I;
+    g.k_stride = 1;
+    g.out_row = J;
+    g.out_col = 1;
+    g.batch = 1;
+  }
+  g.map = tile_map(g);
+  constexpr int64_t most = (int64_t)65535 * 64;  // columns of one launch
+  for (int64_t j0 = 0; j0 < J; j0 += most) {
+    g.R = (int)std::min<int64_t>(J - j0, most);
+    g.inner = mat + j0 * I;
+    g.out = Y + j0 * g.out_col;
+    int bn, bm;
+    choose_tile_unsplit(ctx, g.rows, g.R, g.batch, &bn, &bm);
+    const dim3 grid((unsigned)ceil_div(g.rows, bm),
+                    (unsigned)std::min<int64_t>(g.batch, 65535), (unsigned)ceil_div(g.R, bn));
+    TSR_TRY(dispatch(ctx, s, g, bn, bm, grid));
+  }
+  return TSR_OK;
 }
 
 }  // namespace tsr

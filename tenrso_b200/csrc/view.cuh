@@ -64,6 +64,9 @@ ViewPlan plan_view(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode,
 // Partial sums [splits][I_mode][R] (f: one factor per mode; f[mode] unused).
 int launch_view(tsr_ctx* ctx, cudaStream_t s, const float* X, int ndim, const int64_t* shape,
                 int mode, const float* const* f, int R, const ViewPlan& plan, float* partials);
+// Y[a, j, b] = sum_i mat[j, i] X[a, i, b] for X seen as A x I x B, mat J x I.
+int launch_view_matrix(tsr_ctx* ctx, cudaStream_t s, const float* X, int64_t A, int64_t I,
+                       int64_t B, const float* mat, int64_t J, float* Y);
 void init_view_attributes();
 
 // One translation unit per column-tile width.
