@@ -337,7 +337,8 @@ struct TContract {
   int side_of[kMaxModes];  // output mode -> side
   int pos[kMaxModes];      // output mode -> its index within the side
   int row0[kMaxModes + 1];
-  float* out;
+  float* out[kMaxModes];  // per mode: I_m x R
+  const float* w;         // column scale (R), or null
 };
 
 // Thread (g, r)'s share of M_m[i, r]: groups g < groups split the side's
@@ -396,7 +397,8 @@ __global__ void __launch_bounds__(256) t_contract_kernel(const __grid_constant__
   if (threadIdx.x < R) {
     double t = 0.0;
     for (int q = 0; q < groups; ++q) t += part[q * R + threadIdx.x];
-    c.out[(int64_t)b * R + threadIdx.x] = (float)t;
+    if (c.w) t *= (double)__ldg(c.w + threadIdx.x);
+    c.out[n][(int64_t)(b - c.row0[n]) * R + threadIdx.x] = (float)t;
   }
 }
 
@@ -609,6 +611,35 @@ namespace {
 int reconstruction_grad_device(tsr_ctx* ctx, const float* dG, int ndim, const int64_t* shape,
                                const FactorTable& ft, int R, const float* dw, int precision,
                                float* const* d_out) {
+  // FP32, three or more modes: two passes over G (T and P) and a small
+  // contraction of each instead of one pass per mode, as long as T and P are
+  // no larger than G. 121x95x63x47 rank 24: 4 passes 390 us, this 2.
+  const int64_t total = numel(ndim, shape);
+  if (precision == TSR_PREC_FP32 && ndim >= 3 && R >= 1 && R <= 256 && total > 0) {
+    const int64_t A = prod_range(shape, 0, ndim - 2), C = shape[ndim - 2] * shape[ndim - 1];
+    if (A >= R && C >= R && A <= ((int64_t)1 << 30) && C < INT32_MAX) {
+      void* tp;
+      TSR_TRY(slot_get(ctx, SLOT_MISC1, sizeof(float) * (A + C) * R, &tp));
+      float *T = (float*)tp, *P = T + A * R;
+      TSR_TRY(contract_sides(ctx, dG, ndim, shape, ft.ptr, R, T, P));
+      TContract c{};
+      set_side(c, 0, T, shape, 0, ndim - 2, ft.ptr);
+      set_side(c, 1, P, shape, ndim - 2, ndim, ft.ptr);
+      c.R = R;
+      c.nmodes = ndim;
+      c.w = dw;
+      for (int m = 0; m < ndim; ++m) {
+        c.side_of[m] = m < ndim - 2 ? 0 : 1;
+        c.pos[m] = m < ndim - 2 ? m : m - (ndim - 2);
+        c.row0[m + 1] = c.row0[m] + (int)shape[m];
+        c.out[m] = d_out[m];
+      }
+      t_contract_kernel<<<(unsigned)c.row0[ndim], 256, 0, ctx->stream>>>(c);
+      ctx->launches++;
+      TSR_CUDA(cudaGetLastError());
+      return TSR_OK;
+    }
+  }
   for (int n = 0; n < ndim; ++n) {
     if (shape[n] == 0) continue;
     if (numel(ndim, shape) == 0 || R == 0) {
@@ -1119,7 +1150,7 @@ int tsr_cp_loss_grad_dev_f32(tsr_ctx* ctx, const tsr_dense* X, const float* cons
       c.pos[p] = p;
       c.row0[p + 1] = c.row0[p] + (int)X->shape[p];
     }
-    c.out = (float*)mp;
+    for (int p = 0; p < N - 2; ++p) c.out[p] = (float*)mp + (int64_t)c.row0[p] * R;
     t_contract_kernel<<<(unsigned)lead_rows, 256, 0, ctx->stream>>>(c);
     ctx->launches++;
     TSR_CUDA(cudaGetLastError());
