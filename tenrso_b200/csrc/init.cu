@@ -16,11 +16,13 @@
 // N(0, 0.01) padding columns on stream 500 + n.
 //
 // The singular vectors on the device: the FP64 Gram G = X_(n) X_(n)^T
-// (I_n x I_n; the order of the unfolding's columns does not enter G), then a
-// cyclic Jacobi eigensolver on G in round-robin order (I_n / 2 disjoint
-// rotations per round, each round three launches: rotation angles, row
-// update, column update with the eigenvector update), sweeps until the
-// off-diagonal mass is below 1e-26 of the diagonal's. s_r = sqrt(lambda_r).
+// (I_n x I_n; the order of the unfolding's columns does not enter G), then its
+// leading eigenpairs by tridiagonalisation (modes of up to 160 rows with
+// separated leading eigenvalues), else a cyclic Jacobi eigensolver on G in
+// round-robin order (I_n / 2 disjoint rotations per round, each round three
+// launches: rotation angles, row update, column update with the eigenvector
+// update), sweeps until the off-diagonal mass is below 1e-26 of the
+// diagonal's. s_r = sqrt(lambda_r).
 // v_r (needed by Nnsvd, only through the norms of its positive and negative
 // parts) is X_(n)^T u_r / s_r, formed and reduced on the fly. SVD signs are
 // arbitrary; each u_r is oriented so that its entry of largest magnitude is
@@ -63,47 +65,382 @@ void seeded_normal(uint64_t seed, uint64_t stream, int64_t n, double sigma, doub
 // ---- Gram of an unfolding ---------------------------------------------------
 
 // G[i, i'] = sum_{a, b} X[a, i, b] X[a, i', b], X viewed as A x I x B
-// (A = prod of the modes before n, B = prod after). 32 x 32 output tile per
-// 256-thread CTA (2 x 2 per thread), FP64 accumulation over 32-wide chunks.
+// (A = prod of the modes before n, B = prod after), in FP64 (the products of
+// fp32 values are exact). 64 x 64 output tiles of the upper triangle, 4 x 4
+// per 256-thread CTA, the columns split over blockIdx.y into partial Grams:
+// with one CTA per tile and no split, a 160 x 12288 unfolding occupied 25 of
+// 148 SMs. Bound: shared-memory reads (two operand words per four FMAs).
+constexpr int GR_T = 64, GR_K = 32;
+
 __global__ void __launch_bounds__(256) unfold_gram_kernel(const float* __restrict__ X, int64_t A,
                                                           int64_t I, int64_t B,
-                                                          double* __restrict__ G) {
-  __shared__ double xs[2][32][33];
+                                                          int64_t j_per_split,
+                                                          double* __restrict__ parts) {
+  __shared__ double xs[2][GR_K][GR_T + 1];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t i0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
-  const int64_t J = A * B;
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  for (int64_t j0 = 0; j0 < J; j0 += 32) {
-    // 32 rows x 32 columns of each operand: thread t loads 4 elements each
-    for (int e = threadIdx.x; e < 2 * 32 * 32; e += 256) {
-      const int w = e >> 10, r = (e >> 5) & 31, c = e & 31;
-      const int64_t row = (w ? k0 : i0) + r, j = j0 + c;
-      double v = 0.0;
-      if (row < I && j < J) {
-        const int64_t a = j / B, b = j % B;
-        v = (double)__ldg(X + (a * I + row) * B + b);
-      }
-      xs[w][r][c] = v;
+  // tile pair (ti <= tk) of the upper triangle
+  const int nt = (int)((I + GR_T - 1) / GR_T);
+  int ti = 0, rest = blockIdx.x;
+  while (rest >= nt - ti) rest -= nt - ti++;
+  const int tk = ti + rest;
+  const int64_t i0 = (int64_t)ti * GR_T, k0 = (int64_t)tk * GR_T;
+  const int64_t jb = blockIdx.y * j_per_split, je = min(A * B, jb + j_per_split);
+  const int nop = ti == tk ? 1 : 2;
+  double acc[4][4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[p][q] = 0.0;
+  for (int64_t j0 = jb; j0 < je; j0 += GR_K) {
+    __syncthreads();
+    if (B > 1) {  // lanes along the columns: one (a, b) per thread and step
+      const int c = threadIdx.x & 31;
+      const int64_t j = j0 + c, a = j / B;
+      const float* src = X + a * I * B + (j - a * B);
+      for (int w = 0; w < nop; ++w)
+#pragma unroll
+        for (int q = 0; q < GR_T / 8; ++q) {
+          const int r = (threadIdx.x >> 5) + 8 * q;
+          const int64_t row = (w ? k0 : i0) + r;
+          xs[w][c][r] = row < I && j < je ? (double)__ldg(src + row * B) : 0.0;
+        }
+    } else {  // the last mode: lanes along the rows
+      const int r = threadIdx.x & 63;
+      for (int w = 0; w < nop; ++w)
+#pragma unroll
+        for (int q = 0; q < GR_K / 4; ++q) {
+          const int c = (threadIdx.x >> 6) + 4 * q;
+          const int64_t row = (w ? k0 : i0) + r, j = j0 + c;
+          xs[w][c][r] = row < I && j < je ? (double)__ldg(X + j * I + row) : 0.0;
+        }
     }
     __syncthreads();
-#pragma unroll 8
-    for (int c = 0; c < 32; ++c) {
-      const double x0 = xs[0][ty][c], x1 = xs[0][ty + 16][c];
-      const double y0 = xs[1][tx][c], y1 = xs[1][tx + 16][c];
-      acc[0][0] = fma(x0, y0, acc[0][0]);
-      acc[0][1] = fma(x0, y1, acc[0][1]);
-      acc[1][0] = fma(x1, y0, acc[1][0]);
-      acc[1][1] = fma(x1, y1, acc[1][1]);
+    const double(*ys)[GR_T + 1] = xs[nop - 1];
+#pragma unroll 4
+    for (int c = 0; c < GR_K; ++c) {
+      double x[4], y[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) x[p] = xs[0][c][ty + 16 * p];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = ys[c][tx + 16 * q];
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[p][q] = fma(x[p], y[q], acc[p][q]);
     }
-    __syncthreads();
   }
+  double* G = parts + (int64_t)blockIdx.y * I * I;
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
+  for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
+    for (int q = 0; q < 4; ++q) {
       const int64_t i = i0 + ty + 16 * p, k = k0 + tx + 16 * q;
       if (i < I && k < I) G[i * I + k] = acc[p][q];
     }
+}
+
+// G = the sum of the partial Grams, mirrored from the tiles of the upper
+// triangle. Eight threads share an element, each summing every eighth split.
+__global__ void __launch_bounds__(256) gram_reduce_kernel(const double* __restrict__ parts,
+                                                          int splits, int64_t I,
+                                                          double* __restrict__ G) {
+  const int64_t e = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+  const int g = threadIdx.x & 7;
+  double t = 0.0;
+  if (e < I * I) {
+    const int64_t i = e / I, k = e - i * I;
+    const double* p = parts + (i / GR_T <= k / GR_T ? e : k * I + i);
+    for (int q = g; q < splits; q += 8) t += __ldg(p + q * I * I);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (g == 0 && e < I * I) G[e] = t;
+}
+
+// ---- leading eigenpairs by tridiagonalisation ------------------------------------
+//
+// Householder reduction of G to a tridiagonal T, the leading eigenvalues of T
+// by bisection on Sturm counts, each eigenvector of T from its twisted
+// factorisation (T - lambda I = L D L^T from the top and U D U^T from the
+// bottom, joined at the row with the smallest |gamma|), and the reflections
+// applied back. All FP64. An eigenvector comes out to about eps |T| / gap, so
+// the host takes this path only where the leading eigenvalues are separated by
+// more than 1e-8 of the largest, and the Jacobi solver below otherwise
+// (repeated or zero eigenvalues, non-finite tensors) and beyond kTriRows rows.
+// About 4/3 I^3 operations in three launches for all modes together, against
+// some ten Jacobi sweeps of 6 I^3 in three launches per round each.
+constexpr int kTriRows = 160;
+
+struct TriMode {
+  const double* G;  // I x I
+  int I, k;         // rows, leading pairs wanted
+  double* d;        // I diagonal, then I off-diagonal, then I reflection scales
+  double* V;        // I x I: reflection j in row j, columns j + 1 ..
+  double* lam;      // min(k + 1, I) leading eigenvalues
+  double* U;        // I x k eigenvectors
+};
+struct TriArgs {
+  TriMode m[kMaxModes];
+};
+
+// One CTA per mode, the matrix in registers: warp w holds rows w + 16 a, lane l
+// columns l + 32 b. Three barriers per column; bound by their latency and by
+// the square root and divisions of each reflection.
+template <int RA, int CB>
+__global__ void __launch_bounds__(512, 1) tridiag_kernel(const __grid_constant__ TriArgs g) {
+  constexpr int W = 32 * CB;
+  __shared__ double xr[2][W > 16 * RA ? W : 16 * RA];
+  __shared__ double pb[W > 16 * RA ? W : 16 * RA];
+  __shared__ double part[16][W];
+  __shared__ double dotp[CB];
+  const TriMode& M = g.m[blockIdx.x];
+  const int I = M.I, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double a[RA][CB];
+#pragma unroll
+  for (int ra = 0; ra < RA; ++ra)
+#pragma unroll
+    for (int cb = 0; cb < CB; ++cb) {
+      const int row = w + 16 * ra, col = lane + 32 * cb;
+      a[ra][cb] = row < I && col < I ? M.G[(int64_t)row * I + col] : 0.0;
+    }
+  if (w == 0)
+#pragma unroll
+    for (int cb = 0; cb < CB; ++cb) xr[0][lane + 32 * cb] = a[0][cb];
+  __syncthreads();
+  int buf = 0;
+  for (int j = 0; j < I; ++j, buf ^= 1) {
+    if (threadIdx.x == 0) M.d[j] = xr[buf][j];
+    if (j == I - 1) break;
+    const double x0 = xr[buf][j + 1];
+    double v[CB], ss = 0.0;
+#pragma unroll
+    for (int cb = 0; cb < CB; ++cb) {
+      const int col = lane + 32 * cb;
+      v[cb] = col > j + 1 ? xr[buf][col] : 0.0;
+      ss = fma(v[cb], v[cb], ss);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    double alpha = x0, tau = 0.0, inv = 0.0;
+    if (ss > 0.0) {  // the same in every thread; |x|, 1 + |x0| / |x| and 1 / (x0 - alpha)
+      const double n2 = fma(x0, x0, ss), rn = rsqrt(n2), nrm = n2 * rn;
+      alpha = x0 >= 0.0 ? -nrm : nrm;
+      tau = fma(fabs(x0), rn, 1.0);
+      inv = 1.0 / (x0 - alpha);
+    }
+    if (threadIdx.x == 0) {
+      M.d[I + j] = alpha;
+      M.d[2 * I + j] = tau;
+    }
+    auto v_row = [&](int row) {
+      return row == j + 1 ? 1.0 : row > j + 1 ? xr[buf][row] * inv : 0.0;
+    };
+    double K = 0.0, wl[CB];
+    if (tau != 0.0) {
+      double acc[CB];
+#pragma unroll
+      for (int cb = 0; cb < CB; ++cb) {
+        const int col = lane + 32 * cb;
+        v[cb] = col == j + 1 ? 1.0 : v[cb] * inv;
+        acc[cb] = 0.0;
+        if (w == 0 && col > j && col < I) M.V[(int64_t)j * I + col] = v[cb];
+      }
+#pragma unroll
+      for (int ra = 0; ra < RA; ++ra)
+        if (16 * ra + 15 > j) {
+          const double vr = v_row(w + 16 * ra);
+#pragma unroll
+          for (int cb = 0; cb < CB; ++cb)
+            if (32 * cb + 31 > j) acc[cb] = fma(a[ra][cb], vr, acc[cb]);
+        }
+#pragma unroll
+      for (int cb = 0; cb < CB; ++cb) part[w][lane + 32 * cb] = acc[cb];
+      __syncthreads();
+      if (w < CB) {
+        const int col = threadIdx.x;
+        double p = 0.0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) p += part[q][col];
+        p = col > j ? p * tau : 0.0;
+        pb[col] = p;
+        double dp = p * v_row(col);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dp += __shfl_xor_sync(0xffffffffu, dp, o);
+        if (lane == 0) dotp[w] = dp;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int cb = 0; cb < CB; ++cb) K += dotp[cb];
+      K *= 0.5 * tau;
+#pragma unroll
+      for (int cb = 0; cb < CB; ++cb) wl[cb] = fma(-K, v[cb], pb[lane + 32 * cb]);
+    }
+#pragma unroll
+    for (int ra = 0; ra < RA; ++ra)
+      if (16 * ra + 15 > j) {
+        const int row = w + 16 * ra;
+        if (tau != 0.0) {
+          const double vr = v_row(row), wr = row < W ? fma(-K, vr, pb[row]) : 0.0;
+#pragma unroll
+          for (int cb = 0; cb < CB; ++cb)
+            if (32 * cb + 31 > j) a[ra][cb] = fma(-wr, v[cb], fma(-vr, wl[cb], a[ra][cb]));
+        }
+        if (row == j + 1)
+#pragma unroll
+          for (int cb = 0; cb < CB; ++cb) xr[buf ^ 1][lane + 32 * cb] = a[ra][cb];
+      }
+    __syncthreads();
+  }
+}
+
+// One CTA per wanted eigenvalue and mode (blockIdx.x = r counts them from the
+// largest; r = k gives only the next eigenvalue, for the separation test).
+// Each bisection round tests 256 points at once (8 bits); bound by the serial
+// recurrences over I, a division per row.
+__global__ void __launch_bounds__(256) tri_eigen_kernel(const __grid_constant__ TriArgs g) {
+  __shared__ double d[kTriRows], e[kTriRows], e2[kTriRows];
+  __shared__ double dp[kTriRows], dm[kTriRows], z[kTriRows];
+  __shared__ double lim[2];
+  __shared__ int below;
+  const TriMode& M = g.m[blockIdx.y];
+  const int I = M.I, r = blockIdx.x, t = threadIdx.x;
+  if (r > M.k || r >= I) return;
+  for (int i = t; i < I; i += 256) {
+    d[i] = M.d[i];
+    e[i] = i < I - 1 ? M.d[I + i] : 0.0;
+    e2[i] = e[i] * e[i];
+  }
+  __syncthreads();
+  if (t < 32) {  // Gershgorin bounds
+    double lo = INFINITY, hi = -INFINITY;
+    for (int i = t; i < I; i += 32) {
+      const double rad = fabs(e[i]) + (i > 0 ? fabs(e[i - 1]) : 0.0);
+      lo = fmin(lo, d[i] - rad);
+      hi = fmax(hi, d[i] + rad);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (t == 0) {
+      const double m = fmax(fabs(lo), fabs(hi)) * 4e-16 + 1e-300;
+      lim[0] = lo - m;
+      lim[1] = hi + m;
+    }
+  }
+  __syncthreads();
+  // pivots smaller than this are replaced: they stand for a zero pivot
+  const double piv = fmax(fabs(lim[0]), fabs(lim[1])) * 4.9e-32 + 1e-300;
+  for (int round = 0; round < 7; ++round) {
+    const double lo = lim[0], hi = lim[1];
+    const double x = lo + (hi - lo) * ((t + 1) * (1.0 / 257.0));
+    int above = 0;  // eigenvalues > x: positive pivots of T - x I
+    double q = 1.0;
+    for (int i = 0; i < I; ++i) {
+      q = d[i] - x - (i > 0 ? e2[i - 1] / q : 0.0);
+      if (fabs(q) < piv) q = -piv;
+      above += q > 0.0;
+    }
+    // the points with more than r eigenvalues above them are a prefix
+    const int n = __syncthreads_count(above > r);
+    if (t == n - 1) lim[0] = x;
+    if (t == n) lim[1] = x;
+    __syncthreads();
+  }
+  const double lam = 0.5 * (lim[0] + lim[1]);
+  if (t == 0) M.lam[r] = lam;
+  if (r >= M.k) return;
+  if (t == 0) {
+    double q = 1.0;
+    for (int i = 0; i < I; ++i) {
+      q = d[i] - lam - (i > 0 ? e2[i - 1] / q : 0.0);
+      if (fabs(q) < piv) q = -piv;
+      dp[i] = q;
+    }
+  } else if (t == 32) {
+    double q = 1.0;
+    for (int i = I - 1; i >= 0; --i) {
+      q = d[i] - lam - (i < I - 1 ? e2[i] / q : 0.0);
+      if (fabs(q) < piv) q = -piv;
+      dm[i] = q;
+    }
+  }
+  __syncthreads();
+  if (t < 32) {
+    double best = INFINITY;
+    int at = 0;
+    for (int i = t; i < I; i += 32) {
+      const double gm = fabs(dp[i] + dm[i] - (d[i] - lam));
+      if (gm < best) {
+        best = gm;
+        at = i;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, at, o);
+      if (ob < best || (ob == best && oi < at)) {
+        best = ob;
+        at = oi;
+      }
+    }
+    if (t == 0) below = at;
+  }
+  __syncthreads();
+  const int at = below;
+  for (int i = t; i < I; i += 256)  // step ratios away from the twist
+    z[i] = i < at ? -e[i] / dp[i] : i > at ? -e[i - 1] / dm[i] : 1.0;
+  __syncthreads();
+  if (t == 0) {
+    double q = 1.0;
+    for (int i = at - 1; i >= 0; --i) z[i] = q *= z[i];
+  } else if (t == 32) {
+    double q = 1.0;
+    for (int i = at + 1; i < I; ++i) z[i] = q *= z[i];
+  }
+  __syncthreads();
+  if (t >= 32) return;
+  // normalise, then u = H_0 H_1 .. H_{I-3} z; the next reflection is loaded
+  // while the current one is applied
+  constexpr int N = kTriRows / 32;
+  double u[N], ss = 0.0;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    u[q] = t + 32 * q < I ? z[t + 32 * q] : 0.0;
+    ss = fma(u[q], u[q], ss);
+  }
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const double sc = 1.0 / sqrt(ss);
+#pragma unroll
+  for (int q = 0; q < N; ++q) u[q] *= sc;
+  double v[N], tau = 0.0;
+  auto fetch = [&](int j) {
+    tau = j >= 0 ? M.d[2 * I + j] : 0.0;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const int col = t + 32 * q;
+      v[q] = j >= 0 && col > j && col < I ? M.V[(int64_t)j * I + col] : 0.0;
+    }
+  };
+  fetch(I - 3);
+  for (int j = I - 3; j >= 0; --j) {
+    double cv[N], s = 0.0;
+    const double ct = tau;
+#pragma unroll
+    for (int q = 0; q < N; ++q) cv[q] = v[q];
+    fetch(j - 1);
+    if (ct == 0.0) continue;  // no reflection was stored
+#pragma unroll
+    for (int q = 0; q < N; ++q) s = fma(cv[q], u[q], s);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s *= -ct;
+#pragma unroll
+    for (int q = 0; q < N; ++q) u[q] = fma(s, cv[q], u[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+    if (t + 32 * q < I) M.U[(int64_t)(t + 32 * q) * M.k + r] = u[q];
 }
 
 // ---- cyclic Jacobi (round-robin pairs) ------------------------------------------
@@ -384,10 +721,29 @@ __global__ void svd_factor_kernel(int strategy, const double* __restrict__ Uo, i
   }
 }
 
+// Device scratch of one call: carved from a context slot reserved up front,
+// allocated only past it (the Jacobi solver's matrices).
 struct DevBuf {
   std::vector<void*> ptrs;
+  uint8_t* base = nullptr;
+  size_t left = 0;
+  int reserve(tsr_ctx* ctx, size_t bytes) {
+    void* p;
+    TSR_TRY(slot_get(ctx, SLOT_MISC0, bytes, &p));
+    base = (uint8_t*)p;
+    left = bytes;
+    return TSR_OK;
+  }
+  static size_t room(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
   template <class T>
   int get(T** p, size_t n) {
+    const size_t bytes = room(std::max<size_t>(n, 1) * sizeof(T));
+    if (bytes <= left) {
+      *p = (T*)base;
+      base += bytes;
+      left -= bytes;
+      return TSR_OK;
+    }
     void* q = nullptr;
     cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
     if (e != cudaSuccess)
@@ -474,15 +830,51 @@ int jacobi_eigen(tsr_ctx* ctx, cudaStream_t s, DevBuf& buf, double* G, int I, do
 
 }  // namespace
 
+// The Gram of X's mode-n unfolding (A x I x B) into G.
+static int launch_unfold_gram(tsr_ctx* ctx, cudaStream_t s, const float* X, int64_t A, int64_t I,
+                              int64_t B, double* G) {
+  const int64_t J = A * B, nt = ceil_div(I, GR_T), tiles = nt * (nt + 1) / 2;
+  if (J == 0) {
+    TSR_CUDA(cudaMemsetAsync(G, 0, sizeof(double) * I * I, s));
+    return TSR_OK;
+  }
+  // about four CTAs per SM, at least two chunks each
+  int64_t splits = std::max<int64_t>(1, 4 * (int64_t)ctx->sm_count / tiles);
+  splits = std::min<int64_t>({splits, ceil_div(J, 2 * GR_K), 65535});
+  const int64_t per = round_up(ceil_div(J, splits), GR_K);
+  splits = ceil_div(J, per);
+  void* pp;
+  TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(double) * (size_t)(splits * I * I), &pp));
+  double* parts = (double*)pp;
+  unfold_gram_kernel<<<dim3((unsigned)tiles, (unsigned)splits), 256, 0, s>>>(X, A, I, B, per,
+                                                                             parts);
+  gram_reduce_kernel<<<(unsigned)ceil_div(I * I, 32), 256, 0, s>>>(parts, (int)splits, I, G);
+  ctx->launches += 2;
+  TSR_CUDA(cudaGetLastError());
+  return TSR_OK;
+}
+
+static int launch_tri(tsr_ctx* ctx, cudaStream_t s, const TriArgs& t, int n, int rows, int k) {
+  switch ((rows + 31) / 32) {
+    case 1: tridiag_kernel<2, 1><<<n, 512, 0, s>>>(t); break;
+    case 2: tridiag_kernel<4, 2><<<n, 512, 0, s>>>(t); break;
+    case 3: tridiag_kernel<6, 3><<<n, 512, 0, s>>>(t); break;
+    case 4: tridiag_kernel<8, 4><<<n, 512, 0, s>>>(t); break;
+    default: tridiag_kernel<10, 5><<<n, 512, 0, s>>>(t); break;
+  }
+  tri_eigen_kernel<<<dim3((unsigned)k + 1, (unsigned)n), 256, 0, s>>>(t);
+  ctx->launches += 2;
+  TSR_CUDA(cudaGetLastError());
+  return TSR_OK;
+}
+
 int init_factors_device(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape, int R,
                         int strategy, uint64_t seed, float* d_out) {
   cudaStream_t s = ctx->stream;
-  int64_t off = 0;
-  for (int mode = 0; mode < ndim; ++mode) {
-    const int64_t I = shape[mode];
-    float* out = d_out + off;
-    off += I * R;
-    if (strategy == TSR_INIT_RANDOM || strategy == TSR_INIT_RANDOM_NORMAL) {
+  if (strategy == TSR_INIT_RANDOM || strategy == TSR_INIT_RANDOM_NORMAL) {
+    int64_t off = 0;
+    for (int mode = 0; mode < ndim; ++mode) {
+      const int64_t I = shape[mode];
       std::vector<float> h((size_t)(I * R));
       if (strategy == TSR_INIT_RANDOM) {
         seeded_uniform(seed, 200 + mode, I * R, h.data());
@@ -491,37 +883,101 @@ int init_factors_device(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* 
         seeded_normal(seed, 400 + mode, I * R, 1.0, z.data());
         for (size_t e = 0; e < z.size(); ++e) h[e] = (float)z[e];
       }
-      TSR_CUDA(cudaMemcpyAsync(out, h.data(), sizeof(float) * I * R, cudaMemcpyHostToDevice, s));
+      TSR_CUDA(cudaMemcpyAsync(d_out + off, h.data(), sizeof(float) * I * R,
+                               cudaMemcpyHostToDevice, s));
       TSR_CUDA(cudaStreamSynchronize(s));
-      continue;
+      off += I * R;
     }
-    if (I > kMaxSvdRows)
-      return fail(TSR_E_UNSUPPORTED,
-                  "SVD-based initialisation supports mode sizes up to %d (mode %d has %lld)",
-                  kMaxSvdRows, mode, (long long)I);
-    int64_t A = 1, B = 1;
-    for (int m = 0; m < mode; ++m) A *= shape[m];
-    for (int m = mode + 1; m < ndim; ++m) B *= shape[m];
-    const int64_t J = A * B;
-    DevBuf buf;
-    double* G;
-    TSR_TRY(buf.get(&G, (size_t)(I * I)));
-    dim3 gg((unsigned)ceil_div(I, 32), (unsigned)ceil_div(I, 32));
-    unfold_gram_kernel<<<gg, 256, 0, s>>>(dX, A, I, B, G);
-    ctx->launches++;
-    TSR_CUDA(cudaGetLastError());
-    double* V;
-    int m;
+    return TSR_OK;
+  }
+  // mode n of X as A x I x B, its thin SVD's leading components
+  struct Mode {
+    int64_t A = 1, I = 0, B = 1;
+    int k = 0, m = 0;
+    double *G = nullptr, *V = nullptr;  // Gram; eigenvectors (row stride m)
     std::vector<double> lam;
     std::vector<int> order;
-    TSR_TRY(jacobi_eigen(ctx, s, buf, G, (int)I, &V, &m, &lam, &order));
+    bool ready = false;
+  };
+  std::vector<Mode> ms(ndim);
+  DevBuf buf;
+  size_t bytes = 0;
+  for (int mode = 0; mode < ndim; ++mode) {
+    const size_t I = (size_t)std::min<int64_t>(shape[mode], kMaxSvdRows), r = (size_t)R;
+    // Gram, reflections, vectors, their oriented copy, padding columns, vectors of I or R
+    bytes += sizeof(double) * (2 * I * I + 2 * I * std::min(I, r) + I * r + 3 * I + 7 * r) +
+             16 * 256;
+  }
+  TSR_TRY(buf.reserve(ctx, bytes));
+  TriArgs tri{};
+  int tri_mode[kMaxModes], n_tri = 0, tri_rows = 0, tri_k = 0;
+  size_t lam_off[kMaxModes], lam_n = 0;
+  for (int mode = 0; mode < ndim; ++mode) {
+    Mode& q = ms[mode];
+    q.I = shape[mode];
+    if (q.I > kMaxSvdRows)
+      return fail(TSR_E_UNSUPPORTED,
+                  "SVD-based initialisation supports mode sizes up to %d (mode %d has %lld)",
+                  kMaxSvdRows, mode, (long long)q.I);
+    for (int m = 0; m < mode; ++m) q.A *= shape[m];
+    for (int m = mode + 1; m < ndim; ++m) q.B *= shape[m];
     // the thin SVD of the I x J unfolding has min(I, J) components
-    const int k = (int)std::min<int64_t>(R, std::min<int64_t>(I, J));
+    q.k = (int)std::min<int64_t>(R, std::min<int64_t>(q.I, q.A * q.B));
+    if (q.I == 0) continue;
+    TSR_TRY(buf.get(&q.G, (size_t)(q.I * q.I)));
+    TSR_TRY(launch_unfold_gram(ctx, s, dX, q.A, q.I, q.B, q.G));
+    if (q.I <= kTriRows && q.k > 0) {
+      TriMode& t = tri.m[n_tri];
+      t.G = q.G;
+      t.I = (int)q.I;
+      t.k = q.k;
+      TSR_TRY(buf.get(&t.d, (size_t)(3 * q.I)));
+      TSR_TRY(buf.get(&t.V, (size_t)(q.I * q.I)));
+      TSR_TRY(buf.get(&t.U, (size_t)(q.I * q.k)));
+      lam_off[n_tri] = lam_n;
+      lam_n += (size_t)std::min<int64_t>(q.k + 1, q.I);
+      tri_rows = std::max(tri_rows, t.I);
+      tri_k = std::max(tri_k, t.k);
+      tri_mode[n_tri++] = mode;
+    }
+  }
+  if (n_tri > 0) {
+    double* lam;
+    TSR_TRY(buf.get(&lam, lam_n));
+    for (int t = 0; t < n_tri; ++t) tri.m[t].lam = lam + lam_off[t];
+    TSR_TRY(launch_tri(ctx, s, tri, n_tri, tri_rows, tri_k));
+    std::vector<double> h(lam_n);
+    TSR_CUDA(cudaMemcpyAsync(h.data(), lam, sizeof(double) * lam_n, cudaMemcpyDeviceToHost, s));
+    TSR_CUDA(cudaStreamSynchronize(s));
+    for (int t = 0; t < n_tri; ++t) {
+      Mode& q = ms[tri_mode[t]];
+      const double* l = h.data() + lam_off[t];
+      const int n = (int)std::min<int64_t>(q.k + 1, q.I);
+      bool apart = std::isfinite(l[0]) && l[0] > 0.0;
+      for (int i = 0; i + 1 < n; ++i) apart = apart && l[i] - l[i + 1] > 1e-8 * l[0];
+      if (!apart) continue;
+      q.ready = true;
+      q.V = tri.m[t].U;
+      q.m = q.k;
+      q.lam.assign(l, l + q.k);
+      q.order.resize(q.k);
+      std::iota(q.order.begin(), q.order.end(), 0);
+    }
+  }
+  int64_t off = 0;
+  for (int mode = 0; mode < ndim; ++mode) {
+    Mode& q = ms[mode];
+    const int64_t I = q.I;
+    const int k = q.k;
+    float* out = d_out + off;
+    off += I * R;
+    if (I > 0 && !q.ready)
+      TSR_TRY(jacobi_eigen(ctx, s, buf, q.G, (int)I, &q.V, &q.m, &q.lam, &q.order));
     std::vector<int> col(std::max(k, 1));
     std::vector<double> sv(std::max(k, 1));
     for (int r = 0; r < k; ++r) {
-      col[r] = order[r];
-      sv[r] = std::sqrt(std::max(lam[order[r]], 0.0));
+      col[r] = q.order[r];
+      sv[r] = std::sqrt(std::max(q.lam[q.order[r]], 0.0));
     }
     int* dcol;
     double *dsv, *Uo, *pn, *upn, *dpad;
@@ -541,12 +997,12 @@ int init_factors_device(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* 
                                cudaMemcpyHostToDevice, s));
     }
     if (k > 0) {
-      orient_kernel<<<k, 256, 0, s>>>(V, m, (int)I, dcol, Uo, k, upn);
+      orient_kernel<<<k, 256, 0, s>>>(q.V, q.m, (int)I, dcol, Uo, k, upn);
       ctx->launches++;
       if (strategy == TSR_INIT_NNSVD) {
         const unsigned g = (unsigned)std::max<int64_t>(
-            1, std::min<int64_t>(ceil_div(J, 256), 4 * (int64_t)ctx->sm_count));
-        vnorm_kernel<<<g, 256, sizeof(double) * 64 * 16, s>>>(dX, A, I, B, Uo, k, dsv, pn);
+            1, std::min<int64_t>(ceil_div(q.A * q.B, 256), 4 * (int64_t)ctx->sm_count));
+        vnorm_kernel<<<g, 256, sizeof(double) * 64 * 16, s>>>(dX, q.A, I, q.B, Uo, k, dsv, pn);
         ctx->launches++;
       }
     }
