@@ -184,15 +184,16 @@ struct TriArgs {
 };
 
 // One CTA per mode, the matrix in registers: warp w holds rows w + 16 a, lane l
-// columns l + 32 b. Three barriers per column; bound by their latency and by
-// the square root and divisions of each reflection.
+// columns l + 32 b. Four barriers per column; the reflection and the sums over
+// warps are formed by the CB warps that own a column block (every warp forming
+// them for itself made the kernel instruction-bound, 553 us at 160 rows).
 template <int RA, int CB>
 __global__ void __launch_bounds__(512, 1) tridiag_kernel(const __grid_constant__ TriArgs g) {
-  constexpr int W = 32 * CB;
-  __shared__ double xr[2][W > 16 * RA ? W : 16 * RA];
-  __shared__ double pb[W > 16 * RA ? W : 16 * RA];
-  __shared__ double part[16][W];
-  __shared__ double dotp[CB];
+  constexpr int W = 32 * CB > 16 * RA ? 32 * CB : 16 * RA;
+  __shared__ double xr[2][W];  // the current row of the matrix, the next one
+  __shared__ double vs[W], pb[W];
+  __shared__ double part[16][32 * CB];
+  __shared__ double dotp[CB], scal[1];
   const TriMode& M = g.m[blockIdx.x];
   const int I = M.I, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double a[RA][CB];
@@ -203,6 +204,8 @@ __global__ void __launch_bounds__(512, 1) tridiag_kernel(const __grid_constant__
       const int row = w + 16 * ra, col = lane + 32 * cb;
       a[ra][cb] = row < I && col < I ? M.G[(int64_t)row * I + col] : 0.0;
     }
+  for (int i = threadIdx.x; i < W; i += 512) vs[i] = pb[i] = xr[0][i] = xr[1][i] = 0.0;
+  __syncthreads();
   if (w == 0)
 #pragma unroll
     for (int cb = 0; cb < CB; ++cb) xr[0][lane + 32 * cb] = a[0][cb];
@@ -211,80 +214,94 @@ __global__ void __launch_bounds__(512, 1) tridiag_kernel(const __grid_constant__
   for (int j = 0; j < I; ++j, buf ^= 1) {
     if (threadIdx.x == 0) M.d[j] = xr[buf][j];
     if (j == I - 1) break;
-    const double x0 = xr[buf][j + 1];
-    double v[CB], ss = 0.0;
-#pragma unroll
-    for (int cb = 0; cb < CB; ++cb) {
-      const int col = lane + 32 * cb;
-      v[cb] = col > j + 1 ? xr[buf][col] : 0.0;
-      ss = fma(v[cb], v[cb], ss);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    double alpha = x0, tau = 0.0, inv = 0.0;
-    if (ss > 0.0) {  // the same in every thread; |x|, 1 + |x0| / |x| and 1 / (x0 - alpha)
-      const double n2 = fma(x0, x0, ss), rn = rsqrt(n2), nrm = n2 * rn;
-      alpha = x0 >= 0.0 ? -nrm : nrm;
-      tau = fma(fabs(x0), rn, 1.0);
-      inv = 1.0 / (x0 - alpha);
-    }
-    if (threadIdx.x == 0) {
-      M.d[I + j] = alpha;
-      M.d[2 * I + j] = tau;
-    }
-    auto v_row = [&](int row) {
-      return row == j + 1 ? 1.0 : row > j + 1 ? xr[buf][row] * inv : 0.0;
-    };
-    double K = 0.0, wl[CB];
-    if (tau != 0.0) {
-      double acc[CB];
+    if (w < CB) {
+      // the reflection of x = row j past the diagonal: alpha = -+|x|,
+      // tau = 1 + |x0| / |x|, v = (1, x_i / (x0 - alpha))
+      const double x0 = xr[buf][j + 1];
+      double ss = 0.0;
 #pragma unroll
       for (int cb = 0; cb < CB; ++cb) {
-        const int col = lane + 32 * cb;
-        v[cb] = col == j + 1 ? 1.0 : v[cb] * inv;
-        acc[cb] = 0.0;
-        if (w == 0 && col > j && col < I) M.V[(int64_t)j * I + col] = v[cb];
+        const double x = xr[buf][lane + 32 * cb];
+        if (lane + 32 * cb > j + 1) ss = fma(x, x, ss);
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      double alpha = x0, tau = 0.0, inv = 0.0;
+      if (ss > 0.0) {  // the same in every warp
+        const double n2 = fma(x0, x0, ss), rn = rsqrt(n2), nrm = n2 * rn;
+        alpha = x0 >= 0.0 ? -nrm : nrm;
+        tau = fma(fabs(x0), rn, 1.0);
+        inv = 1.0 / (x0 - alpha);
+      }
+      const int col = threadIdx.x;
+      const double v = col == j + 1 ? 1.0 : col > j + 1 ? xr[buf][col] * inv : 0.0;
+      vs[col] = v;
+      if (tau != 0.0 && col > j && col < I) M.V[(int64_t)j * I + col] = v;
+      if (threadIdx.x == 0) {
+        scal[0] = tau;
+        M.d[I + j] = alpha;
+        M.d[2 * I + j] = tau;
+      }
+    }
+    __syncthreads();
+    const double tau = scal[0];
+    if (tau == 0.0) {  // nothing to reflect: only publish the next row
 #pragma unroll
       for (int ra = 0; ra < RA; ++ra)
-        if (16 * ra + 15 > j) {
-          const double vr = v_row(w + 16 * ra);
+        if (w + 16 * ra == j + 1)
 #pragma unroll
-          for (int cb = 0; cb < CB; ++cb)
-            if (32 * cb + 31 > j) acc[cb] = fma(a[ra][cb], vr, acc[cb]);
-        }
-#pragma unroll
-      for (int cb = 0; cb < CB; ++cb) part[w][lane + 32 * cb] = acc[cb];
+          for (int cb = 0; cb < CB; ++cb) xr[buf ^ 1][lane + 32 * cb] = a[ra][cb];
       __syncthreads();
-      if (w < CB) {
-        const int col = threadIdx.x;
-        double p = 0.0;
+      continue;
+    }
+    // p = tau A v, rows and columns past j
+    double acc[CB];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) p += part[q][col];
-        p = col > j ? p * tau : 0.0;
-        pb[col] = p;
-        double dp = p * v_row(col);
+    for (int cb = 0; cb < CB; ++cb) acc[cb] = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dp += __shfl_xor_sync(0xffffffffu, dp, o);
-        if (lane == 0) dotp[w] = dp;
+    for (int ra = 0; ra < RA; ++ra)
+      if (16 * ra + 15 > j) {
+        const double vr = vs[w + 16 * ra];
+#pragma unroll
+        for (int cb = 0; cb < CB; ++cb) acc[cb] = fma(a[ra][cb], vr, acc[cb]);
       }
-      __syncthreads();
 #pragma unroll
-      for (int cb = 0; cb < CB; ++cb) K += dotp[cb];
-      K *= 0.5 * tau;
+    for (int cb = 0; cb < CB; ++cb) part[w][lane + 32 * cb] = acc[cb];
+    __syncthreads();
+    if (w < CB) {
+      const int col = threadIdx.x;
+      double p0 = 0.0, p1 = 0.0;
 #pragma unroll
-      for (int cb = 0; cb < CB; ++cb) wl[cb] = fma(-K, v[cb], pb[lane + 32 * cb]);
+      for (int q = 0; q < 16; q += 2) {
+        p0 += part[q][col];
+        p1 += part[q + 1][col];
+      }
+      const double p = col > j ? (p0 + p1) * tau : 0.0;
+      pb[col] = p;
+      double dp = p * vs[col];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dp += __shfl_xor_sync(0xffffffffu, dp, o);
+      if (lane == 0) dotp[w] = dp;
+    }
+    __syncthreads();
+    // A -= v w^T + w v^T, w = p - (tau / 2 p.v) v
+    double K = 0.0;
+#pragma unroll
+    for (int cb = 0; cb < CB; ++cb) K += dotp[cb];
+    K *= -0.5 * tau;
+    double vl[CB], wl[CB];
+#pragma unroll
+    for (int cb = 0; cb < CB; ++cb) {
+      vl[cb] = vs[lane + 32 * cb];
+      wl[cb] = fma(K, vl[cb], pb[lane + 32 * cb]);
     }
 #pragma unroll
     for (int ra = 0; ra < RA; ++ra)
       if (16 * ra + 15 > j) {
         const int row = w + 16 * ra;
-        if (tau != 0.0) {
-          const double vr = v_row(row), wr = row < W ? fma(-K, vr, pb[row]) : 0.0;
+        const double vr = -vs[row], wr = fma(K, vr, -pb[row]);
 #pragma unroll
-          for (int cb = 0; cb < CB; ++cb)
-            if (32 * cb + 31 > j) a[ra][cb] = fma(-wr, v[cb], fma(-vr, wl[cb], a[ra][cb]));
-        }
+        for (int cb = 0; cb < CB; ++cb) a[ra][cb] = fma(wr, vl[cb], fma(vr, wl[cb], a[ra][cb]));
         if (row == j + 1)
 #pragma unroll
           for (int cb = 0; cb < CB; ++cb) xr[buf ^ 1][lane + 32 * cb] = a[ra][cb];
