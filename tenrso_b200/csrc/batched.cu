@@ -37,6 +37,7 @@ namespace tsr {
 namespace {
 
 constexpr int kBatchMaxR = 16;
+constexpr size_t kBatchMaxSmem = 200 * 1024;
 
 struct BatchInst {
   int n0, n1, n2, n2p;  // mode sizes; n2p = n2 rounded up to a multiple of 4
@@ -66,6 +67,7 @@ struct BatchArgs {
   int64_t uscratch_floats;
   int* counter;
   int sweeps;
+  int stage_off;     // bytes into the dynamic shared memory (0: no room, see add_rows)
   double tol;
   float ridge_eps;   // f32 epsilon * R * 10 is formed per instance
 };
@@ -194,22 +196,69 @@ __device__ bool solve_mode(const InstSmem& s, const float* M, int rows, int R, i
   return true;
 }
 
-// acc[p][r] += x[p] * W[r] for the four k of x (W: one shared-memory factor
-// row, Rp floats)
+// acc[p] += x[p] * W for the four k of x (W: one shared-memory factor row, Rp
+// floats), as packed fp32 FMAs over column pairs: the same products and sums
+// as scalar FMAs at half the issue slots.
+__device__ __forceinline__ void fma2(uint64_t& d, float x, uint64_t b) {
+  uint64_t xx;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(x));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(xx), "l"(b));
+}
 template <int RQ>
-__device__ __forceinline__ void fma_row4(float (&acc)[4][4 * RQ], const float4 x,
+__device__ __forceinline__ void fma_row4(uint64_t (&acc)[4][2 * RQ], const float4 x,
                                          const float* W) {
-  const float4* w4 = reinterpret_cast<const float4*>(W);
+  const ulonglong2* w2 = reinterpret_cast<const ulonglong2*>(W);
 #pragma unroll
   for (int rq = 0; rq < RQ; ++rq) {
-    const float4 b = w4[rq];
-    const float bb[4] = {b.x, b.y, b.z, b.w};
+    const ulonglong2 b = w2[rq];
+    fma2(acc[0][2 * rq], x.x, b.x);
+    fma2(acc[0][2 * rq + 1], x.x, b.y);
+    fma2(acc[1][2 * rq], x.y, b.x);
+    fma2(acc[1][2 * rq + 1], x.y, b.y);
+    fma2(acc[2][2 * rq], x.z, b.x);
+    fma2(acc[2][2 * rq + 1], x.z, b.y);
+    fma2(acc[3][2 * rq], x.w, b.x);
+    fma2(acc[3][2 * rq + 1], x.w, b.y);
+  }
+}
+template <int RQ>
+__device__ __forceinline__ float acc_at(const uint64_t (&acc)[4][2 * RQ], int p, int r) {
+  const uint64_t v = acc[p][r >> 1];
+  return __uint_as_float((uint32_t)((r & 1) ? v >> 32 : v));
+}
+
+// Adds the items' contributions to their rows of M: v[r] of item t0 + thread
+// belongs to row (t / nkq) % rows. All threads of the CTA call it for the same
+// t0. With `stage` (Rp rows of NT + 1 floats of shared memory) the items meet
+// there and one thread sums each row's run of nkq; without it (instances that
+// fill the shared memory) they add with shared-memory atomics, which a warp's
+// lanes on one row serialise: at 96^3 rank 16 that took most of a pass.
+template <int NT, int Rp>
+__device__ __forceinline__ void add_rows(const float (&v)[Rp], int t0, int items, int nkq,
+                                         int rows, bool split, int R, float* M, float* stage) {
+  const int t = t0 + threadIdx.x;
+  if (!stage) {
+    if (t < items)
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      acc[0][4 * rq + h] = fmaf(x.x, bb[h], acc[0][4 * rq + h]);
-      acc[1][4 * rq + h] = fmaf(x.y, bb[h], acc[1][4 * rq + h]);
-      acc[2][4 * rq + h] = fmaf(x.z, bb[h], acc[2][4 * rq + h]);
-      acc[3][4 * rq + h] = fmaf(x.w, bb[h], acc[3][4 * rq + h]);
+      for (int r = 0; r < Rp; ++r)
+        if (r < R) atomicAdd(M + ((t / nkq) % rows) * Rp + r, v[r]);
+    return;
+  }
+  const int n = min(NT, items - t0);
+  __syncthreads();  // the previous batch of items has been summed
+#pragma unroll
+  for (int r = 0; r < Rp; ++r) stage[r * (NT + 1) + threadIdx.x] = v[r];
+  __syncthreads();
+  const int s0 = t0 / nkq, ns = (t0 + n - 1) / nkq - s0 + 1;
+  for (int e = threadIdx.x; e < ns * Rp; e += NT) {
+    const int r = e % Rp, sg = s0 + e / Rp;
+    const int x0 = max(sg * nkq - t0, 0), x1 = min((sg + 1) * nkq - t0, n);
+    float sum = 0.f;
+    for (int x = x0; x < x1; ++x) sum += stage[r * (NT + 1) + x];
+    if (r < R) {
+      float* m = M + (sg % rows) * Rp + r;
+      if (split) atomicAdd(m, sum);  // other groups of items share the row
+      else *m += sum;
     }
   }
 }
@@ -226,42 +275,48 @@ __device__ __forceinline__ void transpose_c(const InstSmem& s, int n2p, int Rp, 
 // pass 1: M[i, r] += sum_k (sum_j X[i, j, k] B[j, r]) C[k, r]
 template <int NT, int RQ>
 __device__ void pass_v(const float4* __restrict__ X4, int n0, int n1, int nkq, const float* B,
-                       const float* Ct, float* M, int R) {
+                       const float* Ct, float* M, int R, float* stage) {
   constexpr int Rp = 4 * RQ;
   const int nq = n0 * nkq;
   const int split = nq >= NT ? 1 : min(n1, NT / nq);
   const int items = nq * split;
-  for (int t = threadIdx.x; t < items; t += NT) {
-    const int g = t / nq, q = t - g * nq;
-    const int i = q / nkq, kq = q - i * nkq;
-    float acc[4][Rp];
+  for (int t0 = 0; t0 < items; t0 += NT) {
+    const int t = t0 + threadIdx.x;
+    float v[Rp];
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int r = 0; r < Rp; ++r) v[r] = 0.f;
+    if (t < items) {
+      const int g = t / nq, q = t - g * nq;
+      const int i = q / nkq, kq = q - i * nkq;
+      uint64_t acc[4][2 * RQ];
 #pragma unroll
-      for (int r = 0; r < Rp; ++r) acc[p][r] = 0.f;
-    const float4* xp = X4 + (size_t)i * n1 * nkq + kq;
-    // four loads of X in flight per thread, then their FMAs in j order
-    int j = g;
-    for (; j + 3 * split < n1; j += 4 * split) {
-      float4 xs[4];
+      for (int p = 0; p < 4; ++p)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(j + u * split) * nkq);
+        for (int r = 0; r < 2 * RQ; ++r) acc[p][r] = 0;
+      const float4* xp = X4 + (size_t)i * n1 * nkq + kq;
+      // four loads of X in flight per thread, then their FMAs in j order
+      int j = g;
+      for (; j + 3 * split < n1; j += 4 * split) {
+        float4 xs[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], B + (j + u * split) * Rp);
+        for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(j + u * split) * nkq);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], B + (j + u * split) * Rp);
+      }
+      for (; j < n1; j += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)j * nkq), B + j * Rp);
+      // C rows 4kq .. 4kq+3 at column r: one float4 of Ct (lanes read
+      // consecutive float4s; the rows of C would all map to one bank)
+      const float4* Ct4 = reinterpret_cast<const float4*>(Ct);
+#pragma unroll
+      for (int r = 0; r < Rp; ++r) {
+        const float4 c = Ct4[r * nkq + kq];
+        v[r] = fmaf(acc_at<RQ>(acc, 0, r), c.x, 0.f);
+        v[r] = fmaf(acc_at<RQ>(acc, 1, r), c.y, v[r]);
+        v[r] = fmaf(acc_at<RQ>(acc, 2, r), c.z, v[r]);
+        v[r] = fmaf(acc_at<RQ>(acc, 3, r), c.w, v[r]);
+      }
     }
-    for (; j < n1; j += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)j * nkq), B + j * Rp);
-    // C rows 4kq .. 4kq+3 at column r: one float4 of Ct (lanes read
-    // consecutive float4s; the rows of C would all map to one bank)
-    const float4* Ct4 = reinterpret_cast<const float4*>(Ct);
-#pragma unroll
-    for (int r = 0; r < Rp; ++r) {
-      const float4 c = Ct4[r * nkq + kq];
-      float v = fmaf(acc[0][r], c.x, 0.f);
-      v = fmaf(acc[1][r], c.y, v);
-      v = fmaf(acc[2][r], c.z, v);
-      v = fmaf(acc[3][r], c.w, v);
-      if (r < R) atomicAdd(M + i * Rp + r, v);
-    }
+    add_rows<NT, Rp>(v, t0, items, nkq, n0, split > 1, R, M, stage);
   }
 }
 
@@ -269,54 +324,61 @@ __device__ void pass_v(const float4* __restrict__ X4, int n0, int n1, int nkq, c
 // M[j, r] += sum_k U[j, k, r] C[k, r]
 template <int NT, int RQ>
 __device__ void pass_u(const float4* __restrict__ X4, int n0, int n1, int nkq, const float* A,
-                       const float* Ct, float* M, float* U, int R) {
+                       const float* Ct, float* M, float* U, int R, float* stage) {
   constexpr int Rp = 4 * RQ;
   const int nq = n1 * nkq;
   const int split = nq >= NT ? 1 : min(n0, NT / nq);
   const int items = nq * split;
-  for (int t = threadIdx.x; t < items; t += NT) {
-    const int g = t / nq, q = t - g * nq;
-    const int j = q / nkq, kq = q - j * nkq;
-    float acc[4][Rp];
+  for (int t0 = 0; t0 < items; t0 += NT) {
+    const int t = t0 + threadIdx.x;
+    float v[Rp];
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int r = 0; r < Rp; ++r) v[r] = 0.f;
+    if (t < items) {
+      const int g = t / nq, q = t - g * nq;
+      const int j = q / nkq, kq = q - j * nkq;
+      uint64_t acc[4][2 * RQ];
 #pragma unroll
-      for (int r = 0; r < Rp; ++r) acc[p][r] = 0.f;
-    const float4* xp = X4 + (size_t)j * nkq + kq;
-    const size_t istride = (size_t)n1 * nkq;
-    int i = g;
-    for (; i + 3 * split < n0; i += 4 * split) {
-      float4 xs[4];
+      for (int p = 0; p < 4; ++p)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(i + u * split) * istride);
+        for (int r = 0; r < 2 * RQ; ++r) acc[p][r] = 0;
+      const float4* xp = X4 + (size_t)j * nkq + kq;
+      const size_t istride = (size_t)n1 * nkq;
+      int i = g;
+      for (; i + 3 * split < n0; i += 4 * split) {
+        float4 xs[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], A + (i + u * split) * Rp);
-    }
-    for (; i < n0; i += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)i * istride), A + i * Rp);
-    const float4* Ct4 = reinterpret_cast<const float4*>(Ct);
+        for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(i + u * split) * istride);
 #pragma unroll
-    for (int r = 0; r < Rp; ++r) {
-      const float4 c = Ct4[r * nkq + kq];
-      float v = fmaf(acc[0][r], c.x, 0.f);
-      v = fmaf(acc[1][r], c.y, v);
-      v = fmaf(acc[2][r], c.z, v);
-      v = fmaf(acc[3][r], c.w, v);
-      if (r < R) atomicAdd(M + j * Rp + r, v);
-    }
-    // U rows (j, 4kq + p), Rp floats each
+        for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], A + (i + u * split) * Rp);
+      }
+      for (; i < n0; i += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)i * istride), A + i * Rp);
+      const float4* Ct4 = reinterpret_cast<const float4*>(Ct);
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      float4* u4 = reinterpret_cast<float4*>(U + ((size_t)j * (4 * nkq) + 4 * kq + p) * Rp);
+      for (int r = 0; r < Rp; ++r) {
+        const float4 c = Ct4[r * nkq + kq];
+        v[r] = fmaf(acc_at<RQ>(acc, 0, r), c.x, 0.f);
+        v[r] = fmaf(acc_at<RQ>(acc, 1, r), c.y, v[r]);
+        v[r] = fmaf(acc_at<RQ>(acc, 2, r), c.z, v[r]);
+        v[r] = fmaf(acc_at<RQ>(acc, 3, r), c.w, v[r]);
+      }
+      // U rows (j, 4kq + p), Rp floats each
 #pragma unroll
-      for (int rq = 0; rq < RQ; ++rq) {
-        const float4 v = make_float4(acc[p][4 * rq], acc[p][4 * rq + 1], acc[p][4 * rq + 2],
-                                     acc[p][4 * rq + 3]);
-        if (split == 1)
-          u4[rq] = v;
-        else
-          atomicAdd(u4 + rq, v);
+      for (int p = 0; p < 4; ++p) {
+        float4* u4 = reinterpret_cast<float4*>(U + ((size_t)j * (4 * nkq) + 4 * kq + p) * Rp);
+#pragma unroll
+        for (int rq = 0; rq < RQ; ++rq) {
+          const float4 uv =
+              make_float4(acc_at<RQ>(acc, p, 4 * rq), acc_at<RQ>(acc, p, 4 * rq + 1),
+                          acc_at<RQ>(acc, p, 4 * rq + 2), acc_at<RQ>(acc, p, 4 * rq + 3));
+          if (split == 1)
+            u4[rq] = uv;
+          else
+            atomicAdd(u4 + rq, uv);
+        }
       }
     }
+    add_rows<NT, Rp>(v, t0, items, nkq, n1, split > 1, R, M, stage);
   }
 }
 
@@ -329,6 +391,7 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
   const float4* X4 = reinterpret_cast<const float4*>(a.X + in.x_off);
   float* F = a.F + in.f_off;
   float* U = a.uscratch + (size_t)blockIdx.x * a.uscratch_floats;
+  float* stage = a.stage_off ? reinterpret_cast<float*>(smem_raw + a.stage_off) : nullptr;
   __shared__ BatchState st;
   __shared__ int ridge_used;
   if (threadIdx.x == 0) {
@@ -360,7 +423,7 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
     // ---- mode 0
     for (int e = threadIdx.x; e < n0 * Rp; e += NT) s.M[e] = 0.f;
     __syncthreads();
-    pass_v<NT, RQ>(X4, n0, n1, nkq, s.B, s.Ct, s.M, R);
+    pass_v<NT, RQ>(X4, n0, n1, nkq, s.B, s.Ct, s.M, R, stage);
     __syncthreads();
     bool ok = solve_mode<NT>(s, s.M, n0, R, Rp, s.GB, s.GC, s.A, s.GA, ridge_eps, &ridge_used);
     // ---- mode 1
@@ -373,7 +436,7 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
         for (int e = threadIdx.x; e < n4; e += NT) u4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
       __syncthreads();
-      pass_u<NT, RQ>(X4, n0, n1, nkq, s.A, s.Ct, s.M, U, R);
+      pass_u<NT, RQ>(X4, n0, n1, nkq, s.A, s.Ct, s.M, U, R, stage);
       __syncthreads();
       ok = solve_mode<NT>(s, s.M, n1, R, Rp, s.GA, s.GC, s.B, s.GB, ridge_eps, &ridge_used);
     }
@@ -509,11 +572,11 @@ __global__ void batch_reset_kernel(BatchState* st, int n) {
 
 void init_batched_attributes() {
   cudaFuncSetAttribute(batched_als_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+                       (int)kBatchMaxSmem);
   cudaFuncSetAttribute(batched_als_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+                       (int)kBatchMaxSmem);
   cudaFuncSetAttribute(batched_als_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+                       (int)kBatchMaxSmem);
 }
 
 }  // namespace tsr
@@ -549,6 +612,28 @@ struct tsr_batch {
 
 namespace tsr {
 namespace {
+
+// The configuration a new batch starts with (tsr_batch_autotune times them
+// all): one 512-thread CTA per SM, or two of 256. A sweep of an instance of
+// w = n0 n1 n2p (rank padded to 4) takes about 20 us (the solves) + 24 us per
+// 1e6 of w on 512 threads, + 33 us on 256; two CTAs on an SM slow each other's
+// passes by a third. The makespan is that of the largest instance or of the
+// whole batch spread over the slots. Measured: 512 instances of 16..96, 8.9 ms
+// (512 x 1) against 12.1; 300 instances of 8..40, 0.89 against 0.57.
+void initial_config(const tsr_ctx* ctx, const std::vector<BatchInst>& inst, int* threads,
+                    int* ctas_per_sm) {
+  double wmax = 0.0, wsum = 0.0;
+  for (const BatchInst& in : inst) {
+    const double w = 1e-6 * in.n0 * in.n1 * in.n2p * 4 * in.rq;
+    wmax = std::max(wmax, w);
+    wsum += w;
+  }
+  const double n = (double)inst.size(), sms = ctx->sm_count;
+  const double one = std::max(20 + 24 * wmax, (20 * n + 24 * wsum) / sms);
+  const double two = std::max(20 + 33 * wmax, (20 * n + 44 * wsum) / (2 * sms));
+  *threads = one <= two ? 512 : 256;
+  *ctas_per_sm = one <= two ? 1 : 2;
+}
 
 int batch_validate(int n_inst, const int64_t* shapes, const int64_t* ranks) {
   if (n_inst <= 0) return fail(TSR_E_INVALID_ARG, "empty batch");
@@ -642,10 +727,14 @@ int enqueue_run(tsr_ctx* ctx, tsr_batch* bt, int max_iters, double tol, float* d
     a.sweeps = std::min(S, max_iters - l * S);
     a.tol = tol;
     a.ridge_eps = std::numeric_limits<float>::epsilon() * 10.0f;
+    const size_t stage = sizeof(float) * 16 * (bt->threads + 1);
+    const bool room = bt->smem + stage <= kBatchMaxSmem;
+    a.stage_off = room ? (int)bt->smem : 0;
+    const size_t smem = bt->smem + (room ? stage : 0);
     switch (bt->threads) {
-      case 128: batched_als_kernel<128><<<ctas, 128, bt->smem, ctx->stream>>>(a); break;
-      case 512: batched_als_kernel<512><<<ctas, 512, bt->smem, ctx->stream>>>(a); break;
-      default: batched_als_kernel<256><<<ctas, 256, bt->smem, ctx->stream>>>(a); break;
+      case 128: batched_als_kernel<128><<<ctas, 128, smem, ctx->stream>>>(a); break;
+      case 512: batched_als_kernel<512><<<ctas, 512, smem, ctx->stream>>>(a); break;
+      default: batched_als_kernel<256><<<ctas, 256, smem, ctx->stream>>>(a); break;
     }
     ctx->launches++;
     TSR_CUDA(cudaGetLastError());
@@ -773,11 +862,12 @@ int tsr_batch_create_f32(tsr_ctx* ctx, int n_inst, const int64_t* shapes, const 
     work[b] = (double)in.n0 * in.n1 * in.n2p * (4 * in.rq + 4);
   }
   bt->uscratch_floats = (bt->uscratch_floats + 3) / 4 * 4;
+  initial_config(ctx, bt->inst, &bt->threads, &bt->ctas_per_sm);
   auto cleanup = [&](int rc) {
     tsr_batch_destroy(bt);
     return rc;
   };
-  if (bt->smem > 200 * 1024)
+  if (bt->smem > kBatchMaxSmem)
     return cleanup(fail(TSR_E_UNSUPPORTED, "batch instances too large for shared memory"));
   bt->order.resize(n_inst);
   for (int b = 0; b < n_inst; ++b) bt->order[b] = b;
