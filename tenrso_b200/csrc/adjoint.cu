@@ -38,8 +38,9 @@ struct tsr_dense {
   bool d3_three = false;  // the view suits the single-layout 3-way MTTKRP
   bool d3_two = false;    // the view suits the two-sided contraction
   tsr::Dense3 d3{};
-  // FP32 tensors of 3 or more modes: T and P contracted from X seen as an
-  // A x C matrix (A the leading modes' product, C = I_{N-2} I_{N-1})
+  // Tensors of 3 or more modes without that copy: T and P contracted in FP32
+  // from X seen as an A x C matrix (A the leading modes' product, C = I_{N-2}
+  // I_{N-1})
   bool v2_on = false;
   int64_t v2_shape[2] = {0, 0};
 };
@@ -535,6 +536,24 @@ int contract_sides(tsr_ctx* ctx, const float* dX, int N, const int64_t* shape,
   return TSR_OK;
 }
 
+// The four loss scalars and the status word in one read-back into pinned
+// memory and one synchronization.
+int read_scalars(tsr_ctx* ctx, const double* d_scalars, double (&sc)[4]) {
+  void* rb;
+  TSR_TRY(readback_get(ctx, sizeof(sc) + 16, &rb));
+  uint8_t* b = (uint8_t*)rb;
+  TSR_CUDA(cudaMemcpyAsync(b, d_scalars, sizeof(sc), cudaMemcpyDeviceToHost, ctx->stream));
+  TSR_CUDA(cudaMemcpyAsync(b + sizeof(sc), ctx->d_status, sizeof(unsigned),
+                           cudaMemcpyDeviceToHost, ctx->stream));
+  TSR_CUDA(cudaStreamSynchronize(ctx->stream));
+  std::memcpy(sc, b, sizeof(sc));
+  unsigned st;
+  std::memcpy(&st, b + sizeof(sc), sizeof(st));
+  if (st) TSR_TRY(reset_status(ctx));
+  if (st & DS_TIMEOUT) return fail(TSR_E_TIMEOUT, "device wait timed out in the MTTKRP kernel");
+  return TSR_OK;
+}
+
 // Shared validation of tenrso's cp_reconstruct (outer.rs:231-255).
 int validate_reconstruct(int n_factors, const int64_t* fcols, int64_t n_weights, bool has_w) {
   if (n_factors <= 0)
@@ -609,11 +628,13 @@ namespace {
 int reconstruction_grad_device(tsr_ctx* ctx, const float* dG, int ndim, const int64_t* shape,
                                const FactorTable& ft, int R, const float* dw, int precision,
                                float* const* d_out) {
-  // FP32, three or more modes: two passes over G (T and P) and a small
+  // Three or more modes: two FP32 passes over G (T and P) and a small
   // contraction of each instead of one pass per mode, as long as T and P are
-  // no larger than G. 121x95x63x47 rank 24: 4 passes 390 us, this 2.
+  // no larger than G. 121x95x63x47 rank 24: 4 FP32 passes 390 us, this 190. A
+  // BF16x3 request takes it too: G comes new with every call, so each of its N
+  // passes would first write a bf16 unfolding.
   const int64_t total = numel(ndim, shape);
-  if (precision == TSR_PREC_FP32 && ndim >= 3 && R >= 1 && R <= 256 && total > 0) {
+  if (ndim >= 3 && R >= 1 && R <= 256 && total > 0) {
     const int64_t A = prod_range(shape, 0, ndim - 2), C = shape[ndim - 2] * shape[ndim - 1];
     if (A >= R && C >= R && A <= ((int64_t)1 << 30) && C < INT32_MAX) {
       void* tp;
@@ -879,7 +900,9 @@ int tsr_dense_create_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim, cons
     d->d3.hi = (const __nv_bfloat16*)hp;
     d->d3.lo = (const __nv_bfloat16*)lp;
   }
-  if (precision == TSR_PREC_FP32 && ndim >= 3 && vshape[0] <= ((int64_t)1 << 30) &&
+  // (a BF16x3 tensor whose view does not suit the two-sided kernel too: two
+  // FP32 passes against one tensor-core pass per mode)
+  if (!d->d3_on && ndim >= 3 && vshape[0] <= ((int64_t)1 << 30) &&
       vshape[1] * vshape[2] < INT32_MAX) {
     const int64_t v2[2] = {vshape[0], vshape[1] * vshape[2]};
     d->v2_on = true;
@@ -980,10 +1003,9 @@ int tsr_cp_loss_grad_dev_f32(tsr_ctx* ctx, const tsr_dense* X, const float* cons
     ctx->launches++;
     TSR_CUDA(cudaGetLastError());
     if (loss) {
-      TSR_TRY(check_device_status(ctx));
-      TSR_CUDA(cudaMemcpyAsync(loss, X->d_scalars + 2, sizeof(double), cudaMemcpyDeviceToHost,
-                               ctx->stream));
-      TSR_CUDA(cudaStreamSynchronize(ctx->stream));
+      double sc[4];
+      TSR_TRY(read_scalars(ctx, X->d_scalars, sc));
+      *loss = sc[2];
     }
     return TSR_OK;
   };
@@ -1016,10 +1038,8 @@ int tsr_cp_loss_grad_dev_f32(tsr_ctx* ctx, const tsr_dense* X, const float* cons
     ctx->launches++;
     TSR_CUDA(cudaGetLastError());
     if (loss) {
-      TSR_TRY(check_device_status(ctx));
       double sc[4];
-      TSR_CUDA(cudaMemcpyAsync(sc, X->d_scalars, sizeof(sc), cudaMemcpyDeviceToHost, ctx->stream));
-      TSR_CUDA(cudaStreamSynchronize(ctx->stream));
+      TSR_TRY(read_scalars(ctx, X->d_scalars, sc));
       *loss = sc[0] - 2.0 * sc[1] + sc[3];
     }
     return TSR_OK;

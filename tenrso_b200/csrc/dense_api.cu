@@ -169,6 +169,34 @@ static ViewPlan plan_mode_view(const tsr_ctx* ctx, const ModeOperand& op, int R)
   return plan_view(ctx, op.u.ndim, op.shape, op.u.mode, R, op.resident ? ctx->reserve_sms : 0);
 }
 
+// Measured, us per mode with the unfolding (kernel alone), BF16x3 against FP32
+// in place: 301x223x187 rank 32 106-155 (33) against 67-79 (45), rank 128
+// 187-231 (95) against 140-165 (126); 97x83x61x45 rank 32 270-908 (151-366)
+// against 99-123 (73-97), rank 64 (128-246) against (128-161); 128x96x64x48,
+// whose runs suit the run-scaled tensor-core kernel, rank 32 164-1143 (62-114)
+// against 112-140 (86-116), rank 64 167-1173 (65-120) against 185-238
+// (156-215); 40x33x37 any rank (11-27) against (8-10).
+int mttkrp_precision(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
+                     int sweeps, int precision) {
+  if (precision != TSR_PREC_BF16X3 || R > 128) return precision;
+  bool runs = true;  // the run-scaled kernel takes the mode(s)
+  for (int m = 0; m < ndim; ++m)
+    if (mode < 0 || m == mode)
+      runs = runs && plan_tc(ctx, make_unfolding(ndim, shape, m), R).run_length > 0;
+  bool in_place;
+  if (mode >= 0) {
+    in_place = R <= 48 || !runs;
+  } else {
+    // unfoldings written once: FP32 where its kernel is no slower, or by less
+    // than the unfoldings cost over the run (about 7 us per 1e6 elements and
+    // mode, against R / 32 us per sweep)
+    const int64_t n = numel(ndim, shape);
+    in_place = R <= 16 || n * R <= 64000000 || (ndim >= 4 && !runs && R <= 64) ||
+               (int64_t)R * sweeps <= 224;
+  }
+  return in_place ? TSR_PREC_FP32 : precision;
+}
+
 size_t mode_partial_floats(const tsr_ctx* ctx, const ModeOperand& op, int R, int precision) {
   const int64_t splits = precision == TSR_PREC_BF16X3 ? plan_tc(ctx, op.u, R).splits
                                                       : plan_mode_view(ctx, op, R).splits;
@@ -251,6 +279,7 @@ int mttkrp_device(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape,
     TSR_TRY(launch_mttkrp3(ctx, ctx->stream, d, mode, ft, plan, (float*)p, false));
     return launch_mttkrp_reduce(ctx, (float*)p, plan.splits, shape[mode] * R, d_out);
   }
+  precision = mttkrp_precision(ctx, ndim, shape, mode, R, 1, precision);
   ModeOperand op;
   TSR_TRY(prepare_mode(ctx, dX, ndim, shape, mode, precision, 0, &op));
   float* partials;
@@ -371,6 +400,14 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
   }
   const int R = (int)rank;
   const int64_t n = numel(ndim, shape);
+  // 3-way BF16x3: one bf16 hi/lo copy of X read by every mode (no unfoldings)
+  // (the orthonormalisation rewrites a factor after its solve, so the solve's
+  // B image would be stale: that run takes the per-mode operands)
+  const bool d3 = !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
+                  dense3_supported(ndim, shape, R) && ((uintptr_t)dX & 15) == 0 &&
+                  !(cons && cons->orthogonal);
+  if (!sp && !d3)
+    precision = mttkrp_precision(ctx, ndim, shape, -1, R, max_iters, precision);
 
   SweepArgs a;
   std::memset(&a, 0, sizeof(a));  // the bytes of `a` are the graph cache key
@@ -442,16 +479,10 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
   }
   if (a.nonneg) TSR_TRY(launch_clamp_nonneg(ctx, ctx->stream, d_out, ftotal));
 
-  // per-mode unfoldings, resident for the whole run (the reference re-unfolds
+  // per-mode operands, resident for the whole run (the reference re-unfolds
   // in every mttkrp call, mttkrp.rs:126)
   std::vector<ModeOperand> ops(ndim);
   size_t pmax = 0;
-  // 3-way BF16x3: one bf16 hi/lo copy of X read by every mode (no unfoldings)
-  // (the orthonormalisation rewrites a factor after its solve, so the solve's
-  // B image would be stale: that run takes the per-mode unfoldings)
-  const bool d3 = !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
-                  dense3_supported(ndim, shape, R) && ((uintptr_t)dX & 15) == 0 &&
-                  !(cons && cons->orthogonal);
   const bool fused_unfold = !d3 && !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
                             unfold3_supported(ndim, shape);
   if (d3) {
