@@ -285,28 +285,6 @@ __device__ __forceinline__ double gram_loss_part(const double* __restrict__ gram
   return t;
 }
 
-// The Grams of every mode in one launch (pre-zeroed): block b is block
-// b - cta0[m] of mode m, rpc[m] rows each.
-struct GramAll {
-  const float* U[kMaxModes];
-  int64_t rows[kMaxModes];
-  int64_t rpc[kMaxModes];
-  int cta0[kMaxModes + 1];
-  int ndim, R;
-  double* grams;
-};
-
-template <int RB>
-__global__ void __launch_bounds__(256) gram_all_kernel(const __grid_constant__ GramAll g) {
-  __shared__ double Us[kGramChunk * 16 * RB];
-  const int b = blockIdx.x;
-  int m = 0;
-  while (m + 1 < g.ndim && b >= g.cta0[m + 1]) ++m;
-  const int64_t r0 = (int64_t)(b - g.cta0[m]) * g.rpc[m];
-  const int64_t r1 = g.rows[m] < r0 + g.rpc[m] ? g.rows[m] : r0 + g.rpc[m];
-  gram_rows_accumulate<RB>(g.U[m], r0, r1, g.R, g.grams + (int64_t)m * g.R * g.R, Us);
-}
-
 // loss = ||X||^2 - 2 <X, Xhat> + sum_{r,s} prod_n Gram_n[r, s] + reg sum_n tr(Gram_n)
 __global__ void gram_loss_kernel(const double* __restrict__ grams, int ndim, int R, double reg,
                                  double* scal) {
@@ -953,35 +931,8 @@ int tsr_cp_loss_grad_dev_f32(tsr_ctx* ctx, const tsr_dense* X, const float* cons
   TSR_TRY(slot_get(ctx, SLOT_GRAMS, sizeof(double) * N * RR, &gp));
   double* grams = (double*)gp;
   TSR_CUDA(cudaMemsetAsync(X->d_scalars + 1, 0, 2 * sizeof(double), ctx->stream));
-  {
-    // every mode's Gram in one launch
-    TSR_CUDA(cudaMemsetAsync(grams, 0, sizeof(double) * N * RR, ctx->stream));
-    GramAll ga{};
-    ga.ndim = N;
-    ga.R = R;
-    ga.grams = grams;
-    ga.cta0[0] = 0;
-    for (int m = 0; m < N; ++m) {
-      const int64_t rows = X->shape[m];
-      int64_t ctas = std::min<int64_t>(ceil_div(rows, 16), 2 * ctx->sm_count);
-      ga.rpc[m] = ceil_div(rows, ctas);
-      ga.U[m] = d_factors[m];
-      ga.rows[m] = rows;
-      ga.cta0[m + 1] = ga.cta0[m] + (int)ceil_div(rows, ga.rpc[m]);
-    }
-    const unsigned g = (unsigned)ga.cta0[N];
-    switch ((R + 15) / 16) {
-      case 1: gram_all_kernel<1><<<g, 256, 0, ctx->stream>>>(ga); break;
-      case 2: gram_all_kernel<2><<<g, 256, 0, ctx->stream>>>(ga); break;
-      case 3: gram_all_kernel<3><<<g, 256, 0, ctx->stream>>>(ga); break;
-      case 4: gram_all_kernel<4><<<g, 256, 0, ctx->stream>>>(ga); break;
-      case 5: gram_all_kernel<5><<<g, 256, 0, ctx->stream>>>(ga); break;
-      case 6: gram_all_kernel<6><<<g, 256, 0, ctx->stream>>>(ga); break;
-      default: gram_all_kernel<7><<<g, 256, 0, ctx->stream>>>(ga); break;
-    }
-    ctx->launches++;
-    TSR_CUDA(cudaGetLastError());
-  }
+  TSR_CUDA(cudaMemsetAsync(grams, 0, sizeof(double) * N * RR, ctx->stream));
+  TSR_TRY(launch_gram_all(ctx, ctx->stream, N, d_factors, X->shape, R, grams));
   auto grad_of = [&](int n, const float* partials, int splits) -> int {
     const int64_t rows = X->shape[n];
     const int rpc =

@@ -10,6 +10,8 @@
 // ||Xhat||^2 and <X, Xhat> come from the Grams and the last mode's MTTKRP
 // (mathematically identical to the extra mode-0 MTTKRP of helpers.rs:558-579).
 // Grams are stored as their upper triangle (row a, column c >= a).
+#include <algorithm>
+
 #include "als.cuh"
 #include "sm100.cuh"
 
@@ -986,6 +988,95 @@ void init_als_attributes() {
   cudaFuncSetAttribute(solve_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(solve_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   cudaFuncSetAttribute(solve_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+}
+
+namespace {
+// The Grams of every mode in one launch (pre-zeroed): block b is block
+// b - cta0[m] of mode m, rpc[m] rows each.
+struct GramAll {
+  const float* U[kMaxModes];
+  int64_t rows[kMaxModes];
+  int64_t rpc[kMaxModes];
+  int cta0[kMaxModes + 1];
+  int ndim, R;
+  double* grams;
+};
+
+template <int RB>
+__global__ void __launch_bounds__(256) gram_all_kernel(const __grid_constant__ GramAll g) {
+  __shared__ double Us[kGramChunk * 16 * RB];
+  const int b = blockIdx.x;
+  int m = 0;
+  while (m + 1 < g.ndim && b >= g.cta0[m + 1]) ++m;
+  const int64_t r0 = (int64_t)(b - g.cta0[m]) * g.rpc[m];
+  const int64_t r1 = g.rows[m] < r0 + g.rpc[m] ? g.rows[m] : r0 + g.rpc[m];
+  gram_rows_accumulate<RB>(g.U[m], r0, r1, g.R, g.grams + (int64_t)m * g.R * g.R, Us);
+}
+
+
+// Start of a CP-ALS call: the factors copied from `init` (null: already there),
+// the Grams, the state with its history and the status word cleared, in one
+// launch instead of a copy and three memsets, each of which the host enqueues
+// for about as long as the GPU takes for all of them.
+__global__ void als_begin_kernel(const float* __restrict__ init, float* __restrict__ factors,
+                                 int64_t nf, double* __restrict__ grams, int64_t ng,
+                                 double* __restrict__ state, int64_t ns, unsigned* status,
+                                 double* xnorm, double xnorm_value) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  if (init)
+    for (int64_t e = t; e < nf; e += step) factors[e] = __ldg(init + e);
+  for (int64_t e = t; e < ng; e += step) grams[e] = 0.0;
+  for (int64_t e = t; e < ns; e += step)
+    state[e] = state + e == xnorm ? xnorm_value : 0.0;
+  if (t == 0) *status = 0;
+}
+}  // namespace
+
+int launch_als_begin(tsr_ctx* ctx, const float* init, float* factors, int64_t n_factors,
+                     const AlsBuffers& b, int64_t n_grams, size_t state_bytes,
+                     double xnorm_sq) {
+  const int64_t ns = (int64_t)(state_bytes / sizeof(double));
+  const int64_t most = std::max<int64_t>({init ? n_factors : (int64_t)0, n_grams, ns, (int64_t)1});
+  const unsigned grid =
+      (unsigned)std::min<int64_t>(ceil_div(most, 256), 4 * (int64_t)ctx->sm_count);
+  als_begin_kernel<<<grid, 256, 0, ctx->stream>>>(init, factors, n_factors, b.grams, n_grams,
+                                                  (double*)b.state, ns, ctx->d_status,
+                                                  &b.state->xnorm_sq, xnorm_sq);
+  ctx->launches++;
+  TSR_CUDA(cudaGetLastError());
+  return TSR_OK;
+}
+
+int launch_gram_all(tsr_ctx* ctx, cudaStream_t s, int ndim, const float* const* U,
+                    const int64_t* rows, int R, double* grams) {
+  if (R > kMaxRank) return fail(TSR_E_UNSUPPORTED, "rank %d too large", R);
+  GramAll ga{};
+  ga.ndim = ndim;
+  ga.R = R;
+  ga.grams = grams;
+  for (int m = 0; m < ndim; ++m) {
+    const int64_t ctas = std::max<int64_t>(
+        1, std::min<int64_t>(ceil_div(rows[m], 16), 2 * (int64_t)ctx->sm_count));
+    ga.rpc[m] = std::max<int64_t>(1, ceil_div(rows[m], ctas));
+    ga.U[m] = U[m];
+    ga.rows[m] = rows[m];
+    ga.cta0[m + 1] = ga.cta0[m] + (int)ceil_div(rows[m], ga.rpc[m]);
+  }
+  const unsigned g = (unsigned)ga.cta0[ndim];
+  if (g == 0) return TSR_OK;
+  switch ((R + 15) / 16) {
+    case 1: gram_all_kernel<1><<<g, 256, 0, s>>>(ga); break;
+    case 2: gram_all_kernel<2><<<g, 256, 0, s>>>(ga); break;
+    case 3: gram_all_kernel<3><<<g, 256, 0, s>>>(ga); break;
+    case 4: gram_all_kernel<4><<<g, 256, 0, s>>>(ga); break;
+    case 5: gram_all_kernel<5><<<g, 256, 0, s>>>(ga); break;
+    case 6: gram_all_kernel<6><<<g, 256, 0, s>>>(ga); break;
+    default: gram_all_kernel<7><<<g, 256, 0, s>>>(ga); break;
+  }
+  ctx->launches++;
+  TSR_CUDA(cudaGetLastError());
+  return TSR_OK;
 }
 
 int launch_gram(tsr_ctx* ctx, cudaStream_t s, const float* U, int64_t rows, int R,

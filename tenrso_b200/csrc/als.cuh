@@ -117,6 +117,13 @@ void init_als_attributes();
 // Upper triangle of U^T U (FP64) accumulated into gram; zero_first memsets it.
 int launch_gram(tsr_ctx* ctx, cudaStream_t s, const float* U, int64_t rows, int R,
                 double* gram, bool zero_first);
+// Every mode's Gram into grams[m] (pre-zeroed), one launch.
+int launch_gram_all(tsr_ctx* ctx, cudaStream_t s, int ndim, const float* const* U,
+                    const int64_t* rows, int R, double* grams);
+// Factors from init (or null), cleared Grams, state and status word; ||X||^2
+// starts at xnorm_sq.
+int launch_als_begin(tsr_ctx* ctx, const float* init, float* factors, int64_t n_factors,
+                     const AlsBuffers& b, int64_t n_grams, size_t state_bytes, double xnorm_sq);
 // ||X||^2 (FP64) added into *out (which the caller zeroes).
 int launch_norm_sq(tsr_ctx* ctx, cudaStream_t s, const float* X, int64_t n, double* out);
 // Hadamard of all Grams except `mode`, its inverse (ridge retry), and the

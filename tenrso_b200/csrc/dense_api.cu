@@ -439,9 +439,6 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
     a.ft.rows[m] = shape[m];
     ftotal += shape[m] * R;
   }
-  if (d_init != d_out)
-    TSR_CUDA(cudaMemcpyAsync(d_out, d_init, sizeof(float) * ftotal, cudaMemcpyDeviceToDevice,
-                             ctx->stream));
 
   // every buffer is sized before any capture (no allocation inside a graph)
   const int hist_n = std::max(max_iters, 1);
@@ -455,9 +452,9 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
   a.b.ginv = a.b.hadam + (size_t)ndim * R * R;
   a.b.state = (AlsState*)stp;
   a.b.history = (double*)((char*)stp + 256);
-  TSR_CUDA(cudaMemsetAsync(stp, 0, sbytes, ctx->stream));
-  TSR_CUDA(cudaMemsetAsync(gp, 0, gbytes, ctx->stream));
-  TSR_TRY(reset_status(ctx));  // the MTTKRP kernels' status word
+  // (a sparse tensor's sum of squared values was computed when it was built)
+  TSR_TRY(launch_als_begin(ctx, d_init != d_out ? d_init : nullptr, d_out, ftotal, a.b,
+                           (int64_t)(gbytes / sizeof(double)), sbytes, sp ? sp->norm_sq : 0.0));
   const bool tracing = ctx->trace_start != nullptr;
   if (tracing) {  // this call's launches take slots from 0
     ctx->trace_next = 0;
@@ -514,11 +511,20 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
     // of the initial U1 and U2 (the solves rewrite them as the factors change)
     TSR_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
     TSR_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
-    for (int m = 0; m < ndim; ++m)
-      TSR_TRY(launch_gram(ctx, ctx->aux, a.ft.ptr[m], shape[m], R,
-                          a.b.grams + (size_t)m * R * R, false));
-    TSR_TRY(launch_bimage(ctx, ctx->aux, a.ft.ptr[1], d.J, R, d.n_pad, d.bimg[1]));
-    TSR_TRY(launch_bimage(ctx, ctx->aux, a.ft.ptr[2], d.K, R, d.n_pad, d.bimg[2]));
+    TSR_TRY(launch_gram_all(ctx, ctx->aux, ndim, a.ft.ptr, shape, R, a.b.grams));
+    KRImages ki{};
+    ki.n = 2;
+    ki.R = R;
+    ki.n_pad = d.n_pad;
+    for (int w = 0; w < 2; ++w) {
+      KRImage& im = ki.im[w];
+      im.nf = 1;
+      im.U[0] = a.ft.ptr[1 + w];
+      im.size[0] = im.L = (int)shape[1 + w];
+      im.chunks = (int)((w == 0 ? img1 : img2) / 16);
+      im.img = d.bimg[1 + w];
+    }
+    TSR_TRY(launch_kr_images(ctx, ctx->aux, ki));
     TSR_CUDA(cudaEventRecord(ctx->ev[1], ctx->aux));
     TSR_TRY(launch_split_bf16(ctx, ctx->stream, dX, n, (__nv_bfloat16*)hp, (__nv_bfloat16*)lp,
                               &a.b.state->xnorm_sq));
@@ -560,9 +566,7 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
     // ||X||^2 (with the unfoldings, where the fused unfold applies)
     TSR_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
     TSR_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
-    for (int m = 0; m < ndim; ++m)
-      TSR_TRY(launch_gram(ctx, ctx->aux, a.ft.ptr[m], shape[m], R,
-                          a.b.grams + (size_t)m * R * R, false));
+    TSR_TRY(launch_gram_all(ctx, ctx->aux, ndim, a.ft.ptr, shape, R, a.b.grams));
     TSR_CUDA(cudaEventRecord(ctx->ev[1], ctx->aux));
     if (fused_unfold)
       TSR_TRY(launch_unfold3(ctx, dX, shape, uhi, ulo, &a.b.state->xnorm_sq));
@@ -570,14 +574,9 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
       TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
     TSR_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev[1], 0));
   }
-  if (sp)  // sum of squared values, FP64, computed when the tensor was built
-    TSR_CUDA(cudaMemcpyAsync(&a.b.state->xnorm_sq, &sp->norm_sq, sizeof(double),
-                             cudaMemcpyHostToDevice, ctx->stream));
   if (sp || max_iters <= 0) {
     if (!sp) TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
-    for (int m = 0; m < ndim; ++m)
-      TSR_TRY(launch_gram(ctx, ctx->stream, a.ft.ptr[m], shape[m], R,
-                          a.b.grams + (size_t)m * R * R, false));
+    TSR_TRY(launch_gram_all(ctx, ctx->stream, ndim, a.ft.ptr, shape, R, a.b.grams));
   }
 
   const bool time_limited = time_limit_s >= 0.0;
