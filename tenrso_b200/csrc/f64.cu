@@ -2,13 +2,10 @@
 // (crates/tenrso-kernels/src/mttkrp.rs:74-146) and tenrso_decomp::cp_als<f64>
 // (crates/tenrso-decomp/src/cp/core.rs:59-182) with every value in FP64.
 //
-// MTTKRP: M (I_n x R) = X_(n) KR with X viewed as A x I_n x B (A = prod of
-// the modes before n, B = prod after): the unfolding's column j = a B + b is
-// also the forward Khatri-Rao row (mttkrp.rs:182-240), so no unfolding is
-// stored. A CTA owns 32 rows x 64 columns of M and a range of j (split-K);
-// each 32-wide j slice stages its X tile and its Khatri-Rao rows (formed from
-// the factors, one base offset per other mode and j) in shared memory; split
-// partial sums meet in M with FP64 atomics.
+// MTTKRP: the FP64 form of the view kernels (view.cuh): X read in place, the
+// contracted columns in runs of one inner factor, scaled by the product of one
+// row of each other factor. A CTA owns 64 rows x up to 32 columns of M and a
+// range of chunks (split-K); the splits meet in M with FP64 atomics.
 //
 // CP-ALS: the same device state, inverse and fit kernels as the fp32 sweep
 // (als.cu), with an FP64 solve (U = M G^-1, the new Gram and, for the last
@@ -29,81 +26,151 @@ namespace tsr {
 namespace {
 
 struct M64Args {
+  ViewArgs v;  // geometry only
   const double* X;
-  int64_t A, I, B;   // X as A x I x B (the mode's size is I)
-  int R;
-  int n_other;       // modes other than the MTTKRP mode, ascending
-  int64_t osize[kMaxModes];
-  const double* U[kMaxModes];  // their factors (rows x R)
-  int64_t j_per_split;
-  double* M;         // I x R, zeroed by the caller
+  const double* inner;
+  const double* f[kViewOuterMax];
+  const int* done;  // CP-ALS: set once the run has stopped (null: standalone)
+  double* M;        // I x R, zeroed by the caller
 };
 
-constexpr int F64_BI = 32, F64_BC = 64, F64_BJ = 32;
+constexpr int kF64Look = 8;
+constexpr int F64_BM = 64, F64_K = 32, F64_P = F64_K + 1;
 
-__global__ void __launch_bounds__(256) mttkrp_f64_kernel(M64Args g) {
-  __shared__ double xs[F64_BI][F64_BJ + 1];
-  __shared__ double ks[F64_BJ][F64_BC + 1];
-  __shared__ int64_t koff[F64_BJ][kMaxModes];  // row offsets (x R) of each other factor
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  const int64_t i0 = (int64_t)blockIdx.x * F64_BI;
-  const int c0 = blockIdx.y * F64_BC;
-  const int64_t J = g.A * g.B;
-  const int64_t jb = (int64_t)blockIdx.z * g.j_per_split;
-  const int64_t je = min(jb + g.j_per_split, J);
-  double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-  for (int64_t j0 = jb; j0 < je; j0 += F64_BJ) {
-    // per j of the slice: the other modes' indices (row-major over the other
-    // modes in ascending order, i.e. the forward Khatri-Rao row)
-    if (t < F64_BJ) {
-      int64_t j = j0 + t, r = j < je ? j : jb;
-      for (int p = g.n_other - 1; p >= 0; --p) {
-        koff[t][p] = (r % g.osize[p]) * g.R;
-        r /= g.osize[p];
+template <int BN>
+constexpr size_t f64_smem() {
+  return sizeof(double) * 2 * (F64_BM * F64_P + F64_K * BN);
+}
+
+__device__ __forceinline__ void f64_cp8(double* dst, const double* src, bool ok) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = ok ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n)
+               : "memory");
+}
+
+// 4 x 4 outputs per thread (rows ty + 16 i, columns tx + (BN/4) q). Bound by
+// shared-memory reads (two 8-byte words per two FMAs at 4 x 4). The former
+// kernel divided a 64-bit index per element and multiplied 64 columns whatever
+// the rank: 36 us per mode at 120x100x80 rank 24.
+template <int BN>
+__global__ void __launch_bounds__(4 * BN) mttkrp_f64_kernel(const __grid_constant__ M64Args g) {
+  constexpr int TX = BN / 4, NT = 4 * BN, NW = NT / 32;
+  extern __shared__ __align__(16) double sm64[];
+  double* As = sm64;                          // [2][F64_BM][F64_P]
+  double* Bs = sm64 + 2 * F64_BM * F64_P;     // [2][F64_K][BN]
+  if (g.done && *g.done) return;
+  const ViewArgs& v = g.v;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tx = tid % TX, ty = tid / TX;
+  const int64_t i0 = (int64_t)blockIdx.x * F64_BM;
+  const int n0 = blockIdx.z * BN, R = v.R;
+  const int rows_here = (int)min((int64_t)F64_BM, v.rows - i0);
+  const int64_t g0 = (int64_t)blockIdx.y * v.steps_per_split;
+  const int nsteps = (int)min(v.steps_per_split, v.steps - g0);
+  const int bc = tid % BN, bk = tid / BN;  // K's tile: column bc, rows bk, bk + 4, ..
+  const int c = n0 + bc;
+  for (int e = rows_here * F64_P + tid; e < F64_BM * F64_P; e += NT)
+    As[e] = As[F64_BM * F64_P + e] = 0.0;
+
+  const double* X = g.X + i0 * v.row_stride;
+  uint32_t o = (uint32_t)g0 / v.chunks, s0 = ((uint32_t)g0 - o * v.chunks) * v.kc;
+  const double* run = X;
+  double wt = 1.0, braw[F64_K / 4];
+  bool new_run = true;
+  int valid = 0;
+  auto load = [&](int buf) {
+    if (new_run) {
+      run = X;
+      wt = 1.0;
+      uint32_t q = o;
+      for (int p = v.n_outer - 1; p >= 0; --p) {
+        const uint32_t t = p > 0 ? q / v.size[p] : 0, i = q - t * v.size[p];
+        run += i * v.stride[p];
+        if (c < R) wt *= __ldg(g.f[p] + (int64_t)i * R + c);
+        q = t;
+      }
+      new_run = false;
+    }
+    valid = (int)min((uint32_t)v.kc, v.S - s0);
+    double* dst = As + buf * F64_BM * F64_P;
+    if (v.k_stride == 1) {  // lanes along the run
+      const bool in = lane < valid;
+      const double* src = in ? run + s0 + lane + w * v.row_stride : g.X;
+      const int64_t inc = in ? NW * v.row_stride : 0;
+      if (lane < v.kc)
+        for (int m = w; m < rows_here; m += NW) {
+          f64_cp8(dst + m * F64_P + lane, src, in);
+          src += inc;
+        }
+    } else {  // lanes along the rows
+      for (int k = w; k < v.kc; k += NW) {
+        const bool in = k < valid;
+        const double* src = in ? run + (s0 + k) * v.k_stride + lane * v.row_stride : g.X;
+        for (int m = lane; m < rows_here; m += 32) {
+          f64_cp8(dst + m * F64_P + k, src, in);
+          if (in) src += 32 * v.row_stride;
+        }
       }
     }
-    for (int e = t; e < F64_BI * F64_BJ; e += 256) {
-      const int ii = e / F64_BJ, jj = e % F64_BJ;
-      const int64_t i = i0 + ii, j = j0 + jj;
-      double v = 0.0;
-      if (i < g.I && j < je) {
-        const int64_t a = j / g.B, b = j % g.B;
-        v = __ldg(g.X + (a * g.I + i) * g.B + b);
-      }
-      xs[ii][jj] = v;
-    }
-    __syncthreads();
-    for (int e = t; e < F64_BJ * F64_BC; e += 256) {
-      const int jj = e / F64_BC, cc = e % F64_BC;
-      const int c = c0 + cc;
-      double v = 0.0;
-      if (j0 + jj < je && c < g.R) {
-        v = 1.0;
-        for (int p = 0; p < g.n_other; ++p) v *= __ldg(g.U[p] + koff[jj][p] + c);
-      }
-      ks[jj][cc] = v;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int jj = 0; jj < F64_BJ; ++jj) {
-      const double x0 = xs[ty][jj], x1 = xs[ty + 16][jj];
+    const double* ks = g.inner + (int64_t)(s0 + bk) * R + c;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double k = ks[jj][tx + 16 * q];
-        acc[0][q] = fma(x0, k, acc[0][q]);
-        acc[1][q] = fma(x1, k, acc[1][q]);
-      }
+    for (int t = 0; t < F64_K / 4; ++t) {
+      braw[t] = c < R && bk + 4 * t < valid ? __ldg(ks) : 0.0;
+      ks += 4 * R;
     }
+  };
+  auto store_b = [&](int buf) {
+#pragma unroll
+    for (int t = 0; t < F64_K / 4; ++t)
+      Bs[(buf * F64_K + bk + 4 * t) * BN + bc] = bk + 4 * t < valid ? braw[t] * wt : 0.0;
+  };
+  double acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[i][q] = 0.0;
+  load(0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  store_b(0);
+  for (int s = 0; s < nsteps; ++s) {
+    const int buf = s & 1;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+    if (s + 1 < nsteps) {
+      s0 += v.kc;
+      if (s0 >= v.S) {
+        s0 = 0;
+        ++o;
+        new_run = true;
+      }
+      load(buf ^ 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    const double* a = As + buf * F64_BM * F64_P + ty * F64_P;
+    const double* b = Bs + buf * F64_K * BN + tx;
+#pragma unroll 4
+    for (int k = 0; k < v.kc; ++k) {
+      double av[4], bv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) av[i] = a[i * 16 * F64_P + k];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) bv[q] = b[k * BN + TX * q];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[i][q] = fma(av[i], bv[q], acc[i][q]);
+    }
+    if (s + 1 < nsteps) store_b(buf ^ 1);
   }
 #pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    const int64_t i = i0 + ty + 16 * p;
-    if (i >= g.I) continue;
+  for (int i = 0; i < 4; ++i) {
+    const int m = ty + 16 * i;
+    if (m >= rows_here) continue;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int c = c0 + tx + 16 * q;
-      if (c < g.R) atomicAdd(g.M + i * g.R + c, acc[p][q]);
+      const int cc = n0 + tx + TX * q;
+      if (cc < R) atomicAdd(g.M + (i0 + m) * R + cc, acc[i][q]);
     }
   }
 }
@@ -134,14 +201,14 @@ __device__ __forceinline__ void gram_rows(const double* Us, int nr, int R,
 template <int RB>
 __global__ void __launch_bounds__(256)
 solve_f64_kernel(AlsBuffers b, int ndim, int R, int64_t rows, const double* __restrict__ M,
-                 double* __restrict__ U, double* __restrict__ gram, int last) {
+                 double* __restrict__ U, double* __restrict__ gram, int last, int rpc) {
   extern __shared__ __align__(16) double sm[];
   __shared__ double red[16];
   AlsState* st = b.state;
   if (M && st->done) return;
-  constexpr int rpc = 16;
   double* Gi = sm;                    // R x R (solve only)
   double* Us = sm + (M ? R * R : 0);  // rpc x R
+  double* Ms = Us + rpc * R;          // rpc x R (solve only)
   if (M)
     for (int e = threadIdx.x; e < R * R; e += blockDim.x) Gi[e] = b.ginv[e];
   double acc[RB][RB];
@@ -153,16 +220,20 @@ solve_f64_kernel(AlsBuffers b, int ndim, int R, int64_t rows, const double* __re
   for (int64_t r0 = (int64_t)blockIdx.x * rpc; r0 < rows; r0 += (int64_t)gridDim.x * rpc) {
     const int nr = (int)(rows - r0 < rpc ? rows - r0 : rpc);
     __syncthreads();
+    if (M) {
+      for (int e = threadIdx.x; e < nr * R; e += blockDim.x) Ms[e] = M[r0 * R + e];
+      __syncthreads();
+    }
     for (int e = threadIdx.x; e < nr * R; e += blockDim.x) {
       const int64_t g = r0 * R + e;
       double u;
       if (M) {
         const int i = e / R, c = e % R;
-        const double* m = M + (r0 + i) * R;
+        const double* m = Ms + i * R;
         u = 0.0;
         for (int k = 0; k < R; ++k) u = fma(m[k], Gi[k * R + c], u);
         U[g] = u;
-        if (last) ip += M[g] * u;
+        if (last) ip += m[c] * u;
       } else {
         u = U[g];
       }
@@ -221,39 +292,49 @@ unsigned f64_grid(const tsr_ctx* ctx, int64_t n) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), ctx->sm_count * 8));
 }
 
+template <int BN>
+void go_f64(cudaStream_t s, const M64Args& g, dim3 grid) {
+  mttkrp_f64_kernel<BN><<<grid, 4 * BN, f64_smem<BN>(), s>>>(g);
+}
+
 int launch_mttkrp_f64(tsr_ctx* ctx, const double* X, int ndim, const int64_t* shape,
-                      const double* const* U, int R, int mode, double* M) {
+                      const double* const* U, int R, int mode, double* M,
+                      const int* done = nullptr) {
   cudaStream_t s = ctx->stream;
   M64Args g;
   std::memset(&g, 0, sizeof(g));
-  g.X = X;
-  g.A = 1;
-  g.B = 1;
-  for (int m = 0; m < mode; ++m) g.A *= shape[m];
-  for (int m = mode + 1; m < ndim; ++m) g.B *= shape[m];
-  g.I = shape[mode];
-  g.R = R;
-  g.M = M;
+  int64_t J = 1;
   for (int m = 0; m < ndim; ++m)
-    if (m != mode) {
-      g.osize[g.n_other] = shape[m];
-      g.U[g.n_other] = U[m];
-      ++g.n_other;
-    }
-  TSR_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * g.I * R, s));
-  const int64_t J = g.A * g.B;
-  if (g.I == 0 || R == 0 || J == 0) return TSR_OK;
-  const int64_t tiles = ceil_div(g.I, F64_BI) * ceil_div(R, F64_BC);
-  const int64_t want = std::max<int64_t>(1, (4 * (int64_t)ctx->sm_count + tiles - 1) / tiles);
-  const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(want, ceil_div(J, 4 * F64_BJ)));
-  g.j_per_split = round_up(ceil_div(J, splits), F64_BJ);
-  const int64_t nsplit = std::min<int64_t>(ceil_div(J, g.j_per_split), 65535);
-  g.j_per_split = std::max<int64_t>(g.j_per_split, ceil_div(J, nsplit));
-  dim3 grid((unsigned)ceil_div(g.I, F64_BI), (unsigned)ceil_div(R, F64_BC),
-            (unsigned)ceil_div(J, g.j_per_split));
-  if (grid.x > 2147483647u || grid.y > 65535u)
-    return fail(TSR_E_UNSUPPORTED, "f64 MTTKRP grid too large");
-  mttkrp_f64_kernel<<<grid, 256, 0, s>>>(g);
+    if (m != mode) J *= shape[m];
+  TSR_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * shape[mode] * R, s));
+  if (shape[mode] == 0 || R == 0 || J == 0) return TSR_OK;
+  if (J >= (int64_t)UINT32_MAX) return fail(TSR_E_UNSUPPORTED, "unfolding too wide");
+  int inner;
+  describe_view(ndim, shape, mode, &g.v, &inner);
+  g.v.R = R;
+  g.X = X;
+  g.M = M;
+  g.done = done;
+  g.inner = U[inner];
+  for (int m = 0, p = 0; m < ndim; ++m)
+    if (m != mode && m != inner) g.f[p++] = U[m];
+  const int64_t share = ceil_div(R, ceil_div(R, 32));
+  const int bn = share <= 8 ? 8 : share <= 16 ? 16 : share <= 24 ? 24 : 32;
+  const int64_t tiles = ceil_div(g.v.rows, F64_BM) * ceil_div(R, bn);
+  // about three CTAs per SM, at least two chunks each
+  const int64_t want = std::max<int64_t>(
+      1, std::min<int64_t>({3 * (int64_t)ctx->sm_count / tiles, ceil_div(g.v.steps, 2),
+                            (int64_t)65535}));
+  g.v.steps_per_split = ceil_div(g.v.steps, want);
+  dim3 grid((unsigned)ceil_div(g.v.rows, F64_BM),
+            (unsigned)ceil_div(g.v.steps, g.v.steps_per_split), (unsigned)ceil_div(R, bn));
+  if (grid.z > 65535u) return fail(TSR_E_UNSUPPORTED, "f64 MTTKRP grid too large");
+  switch (bn) {
+    case 8: go_f64<8>(s, g, grid); break;
+    case 16: go_f64<16>(s, g, grid); break;
+    case 24: go_f64<24>(s, g, grid); break;
+    default: go_f64<32>(s, g, grid); break;
+  }
   ctx->launches++;
   TSR_CUDA(cudaGetLastError());
   return TSR_OK;
@@ -261,12 +342,16 @@ int launch_mttkrp_f64(tsr_ctx* ctx, const double* X, int ndim, const int64_t* sh
 
 int launch_solve_f64(tsr_ctx* ctx, const AlsBuffers& b, int ndim, int R, int64_t rows,
                      const double* M, double* U, double* gram, bool last) {
+  // 4 rows per step where that still leaves few CTAs (the serial FP64 dot
+  // products set the pace), 16 for tall factors
+  const int rpc = rows <= 8 * (int64_t)ctx->sm_count ? 4 : 16;
   const unsigned grid = (unsigned)std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div(rows, 16), 2 * (int64_t)ctx->sm_count));
-  const size_t smem = sizeof(double) * ((M ? (size_t)R * R : 0) + 16 * (size_t)R);
+      1, std::min<int64_t>(ceil_div(rows, rpc), 2 * (int64_t)ctx->sm_count));
+  const size_t smem = sizeof(double) * ((M ? (size_t)R * R + rpc * (size_t)R : 0) +
+                                        rpc * (size_t)R);
   const int lst = last ? 1 : 0;
 #define TSR_S64(RB) \
-  solve_f64_kernel<RB><<<grid, 256, smem, ctx->stream>>>(b, ndim, R, rows, M, U, gram, lst)
+  solve_f64_kernel<RB><<<grid, 256, smem, ctx->stream>>>(b, ndim, R, rows, M, U, gram, lst, rpc)
   switch ((R + 15) / 16) {
     case 1: TSR_S64(1); break;
     case 2: TSR_S64(2); break;
@@ -295,27 +380,14 @@ void seeded_uniform_f64(uint64_t seed, uint64_t stream, int64_t n, double* out) 
     out[i] = (double)(mix(key + (uint64_t)i * golden) >> 11) * (1.0 / 9007199254740992.0);
 }
 
-struct DevMem {
-  std::vector<void*> p;
-  template <class T>
-  int get(T** q, size_t n) {
-    void* r = nullptr;
-    cudaError_t e = cudaMalloc(&r, std::max<size_t>(n, 1) * sizeof(T));
-    if (e != cudaSuccess)
-      return fail(TSR_E_CUDA, "cudaMalloc (%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
-    p.push_back(r);
-    *q = (T*)r;
-    return TSR_OK;
-  }
-  ~DevMem() {
-    for (void* r : p) cudaFree(r);
-  }
-};
-
 }  // namespace
 
 void init_f64_attributes() {
-  const int big = (int)(sizeof(double) * (kMaxRank * kMaxRank + 16 * kMaxRank));
+  const int big = (int)(sizeof(double) * (kMaxRank * kMaxRank + 32 * kMaxRank));
+  cudaFuncSetAttribute(mttkrp_f64_kernel<24>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)f64_smem<24>());
+  cudaFuncSetAttribute(mttkrp_f64_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)f64_smem<32>());
   cudaFuncSetAttribute(solve_f64_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(solve_f64_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(solve_f64_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -341,12 +413,11 @@ int cp_als_f64_device(tsr_ctx* ctx, const double* dX, int ndim, const int64_t* s
     rmax = std::max<int64_t>(rmax, shape[m]);
   }
   const int hist_n = std::max(max_iters, 1);
-  DevMem mem;
-  double *grams, *Mbuf;
-  void* stp;
-  TSR_TRY(mem.get(&grams, (size_t)(2 * ndim + 1) * R * R));
-  TSR_TRY(mem.get(&Mbuf, (size_t)rmax * R));
-  TSR_TRY(mem.get((uint8_t**)&stp, 256 + sizeof(double) * hist_n));
+  void *gp, *mp, *stp;
+  TSR_TRY(slot_get(ctx, SLOT_GRAMS, sizeof(double) * (size_t)(2 * ndim + 1) * R * R, &gp));
+  TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(double) * (size_t)rmax * R, &mp));
+  TSR_TRY(slot_get(ctx, SLOT_STATE, 256 + sizeof(double) * hist_n, &stp));
+  double *grams = (double*)gp, *Mbuf = (double*)mp;
   AlsBuffers b;
   b.grams = grams;
   b.hadam = grams + (size_t)ndim * R * R;
@@ -373,12 +444,20 @@ int cp_als_f64_device(tsr_ctx* ctx, const double* dX, int ndim, const int64_t* s
     }
     for (int m = 0; m < ndim; ++m) {
       const bool last = m == ndim - 1;
-      TSR_TRY(launch_chol(ctx, s, b, ndim, m, R, ridge, last, tol));
-      TSR_TRY(launch_mttkrp_f64(ctx, dX, ndim, shape, U, R, m, Mbuf));
+      // the inverse runs beside the MTTKRP, as in the fp32 sweep
+      TSR_CUDA(cudaEventRecord(ctx->ev[0], s));
+      TSR_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
+      TSR_TRY(launch_chol(ctx, ctx->aux, b, ndim, m, R, ridge, last, tol));
+      TSR_CUDA(cudaEventRecord(ctx->ev[1], ctx->aux));
+      TSR_TRY(launch_mttkrp_f64(ctx, dX, ndim, shape, U, R, m, Mbuf, &b.state->done));
+      TSR_CUDA(cudaStreamWaitEvent(s, ctx->ev[1], 0));
       TSR_TRY(launch_solve_f64(ctx, b, ndim, R, shape[m], Mbuf, const_cast<double*>(U[m]),
                                grams + (size_t)m * R * R, last));
     }
-    // the fit of this sweep, then the stop decision on the host
+    // the next sweep's first inverse forms this sweep's fit and decides whether
+    // to stop; every kernel after a stop returns at once, so the host looks
+    // only every kF64Look sweeps (and each sweep under a time limit)
+    if (time_limit_s < 0.0 && (iter + 1) % kF64Look != 0) continue;
     TSR_TRY(launch_fit(ctx, s, b, ndim, R, tol));
     AlsState hs;
     TSR_CUDA(cudaMemcpyAsync(&hs, b.state, sizeof(hs), cudaMemcpyDeviceToHost, s));
@@ -390,9 +469,15 @@ int cp_als_f64_device(tsr_ctx* ctx, const double* dX, int ndim, const int64_t* s
                   (double)ridge);
     if (hs.done) break;
   }
+  if (max_iters > 0) TSR_TRY(launch_fit(ctx, s, b, ndim, R, tol));
   AlsState hs;
   TSR_CUDA(cudaMemcpyAsync(&hs, b.state, sizeof(hs), cudaMemcpyDeviceToHost, s));
   TSR_CUDA(cudaStreamSynchronize(s));
+  if (hs.status & DS_NOT_SPD)
+    return fail(TSR_E_NOT_SPD,
+                "Linear algebra error: Gram matrix is not positive definite (ridge %g also "
+                "failed)",
+                (double)ridge);
   if (info) {
     info->fit = hs.fit;
     // core.rs:116-124: the time check comes before the sweep is counted
@@ -427,13 +512,13 @@ int tsr_mttkrp_f64(tsr_ctx* ctx, const double* tensor, int ndim, const int64_t* 
   TSR_TRY(check_ctx(ctx));
   const int R = (int)factor_cols[0];
   const int64_t n = numel(ndim, shape);
-  DevMem mem;
-  double *dX, *dF, *dM;
   int64_t ftotal = 0;
   for (int m = 0; m < ndim; ++m) ftotal += shape[m] * R;
-  TSR_TRY(mem.get(&dX, (size_t)n));
-  TSR_TRY(mem.get(&dF, (size_t)ftotal));
-  TSR_TRY(mem.get(&dM, (size_t)shape[mode] * R));
+  void *xp, *fp, *mp;
+  TSR_TRY(slot_get(ctx, SLOT_TENSOR, sizeof(double) * std::max<int64_t>(n, 1), &xp));
+  TSR_TRY(slot_get(ctx, SLOT_FACTORS, sizeof(double) * std::max<int64_t>(ftotal, 1), &fp));
+  TSR_TRY(slot_get(ctx, SLOT_OUT, sizeof(double) * std::max<int64_t>(shape[mode] * R, 1), &mp));
+  double *dX = (double*)xp, *dF = (double*)fp, *dM = (double*)mp;
   TSR_CUDA(cudaMemcpyAsync(dX, tensor, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   const double* U[kMaxModes];
   int64_t off = 0;
@@ -482,10 +567,10 @@ int tsr_cp_als_f64(tsr_ctx* ctx, const double* tensor, int ndim, const int64_t* 
     }
     init = init_buf.data();
   }
-  DevMem mem;
-  double *dX, *dF;
-  TSR_TRY(mem.get(&dX, (size_t)n));
-  TSR_TRY(mem.get(&dF, (size_t)ftotal));
+  void *xp, *fp;
+  TSR_TRY(slot_get(ctx, SLOT_TENSOR, sizeof(double) * std::max<int64_t>(n, 1), &xp));
+  TSR_TRY(slot_get(ctx, SLOT_FACTORS, sizeof(double) * std::max<int64_t>(ftotal, 1), &fp));
+  double *dX = (double*)xp, *dF = (double*)fp;
   TSR_CUDA(cudaMemcpyAsync(dX, tensor, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   TSR_CUDA(cudaMemcpyAsync(dF, init, sizeof(double) * ftotal, cudaMemcpyHostToDevice,
                            ctx->stream));

@@ -83,7 +83,9 @@ void choose_tile_unsplit(const tsr_ctx* ctx, int64_t rows, int64_t R, int64_t ba
 // a chunk is contiguous in memory (or, for the last mode's MTTKRP, its rows
 // are); one shorter than half a chunk would leave most of each step empty, so
 // then it is the longest one.
-void describe(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner) {
+}  // namespace
+
+void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner) {
   int64_t stride[kMaxModes], st = 1;
   for (int m = ndim - 1; m >= 0; --m) {
     stride[m] = st;
@@ -113,6 +115,7 @@ void describe(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner)
   g->steps = runs * g->chunks;
 }
 
+namespace {
 int tile_map(const ViewArgs& g) {
   if (g.k_stride != 1) return g.row_stride == 1 ? VIEW_ACROSS : VIEW_STRIDED;
   bool vec = ((uintptr_t)g.X & 15) == 0 && g.S % 4 == 0 && g.row_stride % 4 == 0 &&
@@ -140,7 +143,7 @@ ViewPlan plan_view(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode,
   std::memset(&g, 0, sizeof(g));
   int inner;
   choose_tile(shape[mode], R, &p.bn, &p.bm);
-  describe(ndim, shape, mode, &g, &inner);
+  describe_view(ndim, shape, mode, &g, &inner);
   const int per_sm = std::max(1, g_ctas[width_index(p.bn)][rows_index(p.bm)]);
   const int64_t tiles = ceil_div(g.rows, p.bm) * ceil_div(R, p.bn);
   const int64_t slots = (int64_t)std::max(1, ctx->sm_count - reserve) * per_sm;
@@ -159,7 +162,7 @@ int launch_view(tsr_ctx* ctx, cudaStream_t s, const float* X, int ndim, const in
   ViewArgs g;
   std::memset(&g, 0, sizeof(g));
   int inner;
-  describe(ndim, shape, mode, &g, &inner);
+  describe_view(ndim, shape, mode, &g, &inner);
   int64_t cols = 1;
   for (int m = 0; m < ndim; ++m)
     if (m != mode) cols *= shape[m];

@@ -57,6 +57,9 @@ struct ViewPlan {
   int64_t steps_per_split = 0;
 };
 
+// The geometry of one mode's contraction (rows, strides, runs, chunks, outer
+// modes) and its inner mode; element-type independent.
+void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner);
 // The MTTKRP of X (row-major, `shape`) for `mode`, R columns; `reserve`: SMs
 // the plan leaves to other kernels.
 ViewPlan plan_view(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
