@@ -391,7 +391,6 @@ int cp_als_accelerated_device(tsr_ctx* ctx, const float* dX, int ndim, const int
   // operand per mode
   const bool d3 = precision == TSR_PREC_BF16X3 && dense3_supported(ndim, shape, R) &&
                   ((uintptr_t)dX & 15) == 0;
-  if (!d3) precision = mttkrp_precision(ctx, ndim, shape, -1, R, max_iters, precision);
   Dense3 d;
   std::memset(&d, 0, sizeof(d));
   std::vector<ModeOperand> ops(ndim);

@@ -44,10 +44,11 @@ int prepare_mode(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape, 
                  int precision, int slot_index, ModeOperand* op);
 // The precision in which a requested BF16x3 MTTKRP off the single-layout path
 // runs: FP32 where reading X in place beats writing and reading bf16
-// unfoldings (FP32 is then also the more accurate). mode < 0: every mode, once
-// per sweep of an ALS run of `sweeps` on unfoldings written once.
+// unfoldings (FP32 is then also the more accurate). For single calls: an ALS
+// run writes its unfoldings once, and its iterations amplify the rounding of
+// whichever precision it takes, so it takes the one that it was given.
 int mttkrp_precision(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
-                     int sweeps, int precision);
+                     int precision);
 // Partial floats run_mttkrp_partials will need for this operand.
 size_t mode_partial_floats(const tsr_ctx* ctx, const ModeOperand& op, int R, int precision);
 // Split-K partial MTTKRP of one mode into the context's partial slot.

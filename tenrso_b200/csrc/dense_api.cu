@@ -177,24 +177,10 @@ static ViewPlan plan_mode_view(const tsr_ctx* ctx, const ModeOperand& op, int R)
 // against 112-140 (86-116), rank 64 167-1173 (65-120) against 185-238
 // (156-215); 40x33x37 any rank (11-27) against (8-10).
 int mttkrp_precision(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
-                     int sweeps, int precision) {
+                     int precision) {
   if (precision != TSR_PREC_BF16X3 || R > 128) return precision;
-  bool runs = true;  // the run-scaled kernel takes the mode(s)
-  for (int m = 0; m < ndim; ++m)
-    if (mode < 0 || m == mode)
-      runs = runs && plan_tc(ctx, make_unfolding(ndim, shape, m), R).run_length > 0;
-  bool in_place;
-  if (mode >= 0) {
-    in_place = R <= 48 || !runs;
-  } else {
-    // unfoldings written once: FP32 where its kernel is no slower, or by less
-    // than the unfoldings cost over the run (about 7 us per 1e6 elements and
-    // mode, against R / 32 us per sweep)
-    const int64_t n = numel(ndim, shape);
-    in_place = R <= 16 || n * R <= 64000000 || (ndim >= 4 && !runs && R <= 64) ||
-               (int64_t)R * sweeps <= 224;
-  }
-  return in_place ? TSR_PREC_FP32 : precision;
+  const bool runs = plan_tc(ctx, make_unfolding(ndim, shape, mode), R).run_length > 0;
+  return R <= 48 || !runs ? TSR_PREC_FP32 : precision;
 }
 
 size_t mode_partial_floats(const tsr_ctx* ctx, const ModeOperand& op, int R, int precision) {
@@ -279,7 +265,7 @@ int mttkrp_device(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* shape,
     TSR_TRY(launch_mttkrp3(ctx, ctx->stream, d, mode, ft, plan, (float*)p, false));
     return launch_mttkrp_reduce(ctx, (float*)p, plan.splits, shape[mode] * R, d_out);
   }
-  precision = mttkrp_precision(ctx, ndim, shape, mode, R, 1, precision);
+  precision = mttkrp_precision(ctx, ndim, shape, mode, R, precision);
   ModeOperand op;
   TSR_TRY(prepare_mode(ctx, dX, ndim, shape, mode, precision, 0, &op));
   float* partials;
@@ -406,8 +392,6 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
   const bool d3 = !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
                   dense3_supported(ndim, shape, R) && ((uintptr_t)dX & 15) == 0 &&
                   !(cons && cons->orthogonal);
-  if (!sp && !d3)
-    precision = mttkrp_precision(ctx, ndim, shape, -1, R, max_iters, precision);
 
   SweepArgs a;
   std::memset(&a, 0, sizeof(a));  // the bytes of `a` are the graph cache key
