@@ -253,8 +253,14 @@ __device__ __forceinline__ void add_rows(const float (&v)[Rp], int t0, int items
   for (int e = threadIdx.x; e < ns * Rp; e += NT) {
     const int r = e % Rp, sg = s0 + e / Rp;
     const int x0 = max(sg * nkq - t0, 0), x1 = min((sg + 1) * nkq - t0, n);
-    float sum = 0.f;
-    for (int x = x0; x < x1; ++x) sum += stage[r * (NT + 1) + x];
+    const float* p = stage + r * (NT + 1);
+    float s4[4] = {0.f, 0.f, 0.f, 0.f};  // four short chains: less latency and rounding
+    int x = x0;
+    for (; x + 3 < x1; x += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s4[u] += p[x + u];
+    for (; x < x1; ++x) s4[0] += p[x];
+    const float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
     if (r < R) {
       float* m = M + (sg % rows) * Rp + r;
       if (split) atomicAdd(m, sum);  // other groups of items share the row
