@@ -112,9 +112,13 @@ int flush_l2(tsr_ctx* ctx, cudaStream_t s) {
 }
 
 int read_status(tsr_ctx* ctx, unsigned* out) {
-  TSR_CUDA(cudaMemcpyAsync(out, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost,
+  // into pinned memory: a copy to the caller's stack would be staged
+  void* rb;
+  TSR_TRY(readback_get(ctx, sizeof(unsigned), &rb));
+  TSR_CUDA(cudaMemcpyAsync(rb, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost,
                            ctx->stream));
   TSR_CUDA(cudaStreamSynchronize(ctx->stream));
+  *out = *(const unsigned*)rb;
   return TSR_OK;
 }
 

@@ -190,7 +190,7 @@ mttkrp_f32_splitk_kernel(const float* __restrict__ A, int64_t rows, int64_t K, i
 
 // out[e] = sum over splits of partials[s][e] (FP64), optionally times w[e % R].
 // `groups` threads share an element, each summing every groups-th split with
-// four loads in flight; the groups combine through shared memory.
+// eight loads in flight; the groups combine through shared memory.
 __global__ void __launch_bounds__(256)
 mttkrp_reduce_kernel(const float* __restrict__ partials, int splits, int64_t n, int groups,
                      int R, const float* __restrict__ w, float* __restrict__ out) {
@@ -202,12 +202,16 @@ mttkrp_reduce_kernel(const float* __restrict__ partials, int splits, int64_t n, 
   if (k < n) {
     const float* p = partials + k;
     int q = g;
-    for (; q + 3 * groups < splits; q += 4 * groups) {
-      const float v0 = __ldg(p + (int64_t)q * n);
-      const float v1 = __ldg(p + (int64_t)(q + groups) * n);
-      const float v2 = __ldg(p + (int64_t)(q + 2 * groups) * n);
-      const float v3 = __ldg(p + (int64_t)(q + 3 * groups) * n);
-      s += ((double)v0 + (double)v1) + ((double)v2 + (double)v3);
+    for (; q + 7 * groups < splits; q += 8 * groups) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = __ldg(p + (int64_t)(q + u * groups) * n);
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) s += (double)v[u] + (double)v[u + 1];
+    }
+    for (; q + groups < splits; q += 2 * groups) {
+      const float v0 = __ldg(p + (int64_t)q * n), v1 = __ldg(p + (int64_t)(q + groups) * n);
+      s += (double)v0 + (double)v1;
     }
     for (; q < splits; q += groups) s += (double)__ldg(p + (int64_t)q * n);
   }
@@ -307,10 +311,11 @@ int launch_mttkrp_reduce_scaled(tsr_ctx* ctx, const float* partials, int splits,
   if (n == 0) return TSR_OK;
   // enough threads per element that a small result with many splits still
   // fills the SMs (32 groups leave 8 consecutive elements, one 32-byte sector,
-  // per group); beyond 8 groups only while the grid is short of 4 CTAs per SM
+  // per group), and no more: with 393216 elements of 6 splits, four groups
+  // took 13.5 us, one 6
   int groups = 1;
   while (groups < 32 && 2 * groups <= splits &&
-         (groups < 8 || ceil_div(n * groups, 256) < 4 * (int64_t)ctx->sm_count))
+         ceil_div(n * groups, 256) < 4 * (int64_t)ctx->sm_count)
     groups *= 2;
   const int per = 256 / groups;
   mttkrp_reduce_kernel<<<(unsigned)ceil_div(n, per), 256, 0, ctx->stream>>>(
