@@ -1,0 +1,70 @@
+"""Branches that only some inputs reach: the eigensolvers behind the SVD start
+and the row sums of the batched CP-ALS."""
+import numpy as np
+import pytest
+
+import tenrso_b200 as tb
+
+pytestmark = pytest.mark.gpu
+
+
+def unfold(X, m):
+    return np.moveaxis(X.astype(np.float64), m, 0).reshape(X.shape[m], -1)
+
+
+# tridiagonalisation up to 160 rows, Jacobi rotations beyond and where leading
+# eigenvalues coincide; one row, more columns asked for than rows of the Gram
+# are independent
+@pytest.mark.parametrize("kind,shape,R", [
+    ("normal", (160, 9, 31), 16), ("normal", (161, 9, 31), 16), ("normal", (33, 2, 40), 2),
+    ("normal", (1, 12, 30), 1), ("equal", (24, 24, 1), 6), ("rank1", (40, 21, 17), 1),
+    ("huge", (20, 30, 11), 5), ("tiny", (20, 30, 11), 5)])
+def test_svd_start(kind, shape, R):
+    """Each factor column is a unit eigenvector of X_(n) X_(n)^T: FP64 vectors
+    rounded to FP32 (6e-8 per entry), so the residual is at most 1e-6 of the
+    largest eigenvalue and the columns are orthonormal to 1e-6; the values are
+    the leading ones to 1e-6."""
+    rng = np.random.default_rng(len(kind) + sum(shape))
+    if kind == "equal":  # an orthogonal matrix: every singular value is 1
+        X = np.linalg.qr(rng.standard_normal(shape[:2]))[0].reshape(shape)
+    elif kind == "rank1":
+        X = np.einsum("i,j,k->ijk", *[rng.standard_normal(n) for n in shape])
+    else:
+        X = rng.standard_normal(shape) * {"normal": 1.0, "huge": 1e15, "tiny": 1e-15}[kind]
+    X = X.astype(np.float32)
+    for m, F in enumerate(tb.initialize_factors(X, R, "svd", seed=3)):
+        G = unfold(X, m) @ unfold(X, m).T
+        lam = np.linalg.eigvalsh(G)[::-1]
+        F = F.astype(np.float64)
+        k = min(R, shape[m], X.size // shape[m])
+        V = F[:, :k]
+        assert np.abs(V.T @ V - np.eye(k)).max() <= 1e-6, m
+        val = np.einsum("ir,ij,jr->r", V, G, V)
+        assert np.abs(val - lam[:k]).max() <= 1e-6 * lam[0], m
+        assert np.linalg.norm(G @ V - V * val, axis=0).max() <= 1e-6 * lam[0], m
+
+
+@pytest.mark.parametrize("threads,cps", [(128, 4), (256, 2), (512, 1)])
+@pytest.mark.parametrize("long", [0, 5900])
+def test_batched_row_sums(orc, threads, cps, long):
+    """Items that meet in shared memory, and (with an instance that fills it)
+    atomic sums; several groups per row, rows that straddle a block of items,
+    one-element modes. The fit after ten sweeps to 1e-4 of the FP64 one."""
+    shapes = [((5, 4, 3), 2), ((2, 70, 90), 2), ((40, 3, 17), 3), ((96, 33, 61), 16),
+              ((1, 9, 30), 1)] + ([((4, long, 8), 4)] if long else [])
+    rng = np.random.default_rng(9)
+    Xs, inits = [], []
+    for s, R in shapes:
+        fs = [rng.random((n, R)) + 0.1 for n in s]
+        X = np.einsum("ir,jr,kr->ijk", *fs)
+        X += 0.05 * np.linalg.norm(X) / np.sqrt(X.size) * rng.standard_normal(s)
+        Xs.append(X.astype(np.float32))
+        inits.append([rng.random((n, R)).astype(np.float32) for n in s])
+    b = tb.BatchedCpAls(Xs, [R for _, R in shapes])
+    b.set_config(threads, 0, cps)
+    for X, (s, R), init, r in zip(Xs, shapes, inits, b.cp_als(10, 0.0, init=inits)):
+        _, info = orc.cp_als(X.astype(np.float64), R, 10, 0.0,
+                             [f.astype(np.float64) for f in init])
+        assert r.iters == info["iters"]
+        assert abs(r.fit - info["fit"]) <= 1e-4, (s, R)
+    b.close()

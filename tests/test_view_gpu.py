@@ -1,0 +1,159 @@
+"""The kernels that read a row-major tensor in place: MTTKRP in FP32 and FP64,
+n-mode products, the two-pass reconstruction gradient, and the FP32 route of
+BF16x3 requests, at the sizes where their tiles, runs and load patterns change.
+
+Tolerances against FP64, relative Frobenius: FP32 sums of N(0,1) products, in
+chains of 16 columns or of at most 130 terms, 1e-5 (the bound of the other FP32
+MTTKRP tests); BF16x3 1e-4; FP64 1e-12; reconstruction, at most 66 products per
+entry, 1e-6."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import tenrso_b200 as tb
+from tenrso_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    b = np.asarray(b, np.float64)
+    return np.linalg.norm(np.asarray(a, np.float64) - b) / max(np.linalg.norm(b), 1e-300)
+
+
+def mttkrp64(X, fs, mode):
+    kr = np.ones((1, fs[0].shape[1]))
+    for m, f in enumerate(fs):
+        if m != mode:
+            kr = (kr[:, None, :] * f.astype(np.float64)[None]).reshape(-1, kr.shape[1])
+    return np.moveaxis(X.astype(np.float64), mode, 0).reshape(X.shape[mode], -1) @ kr
+
+
+def device(a, offset=0):
+    """A copy of `a` on the GPU that starts `offset` elements into its buffer."""
+    import torch
+    buf = torch.empty(a.size + offset, dtype=torch.float32, device="cuda")
+    t = buf[offset:].reshape(a.shape)
+    t.copy_(torch.from_numpy(a))
+    return t
+
+
+def draw(shape, R, seed=7):
+    rng = np.random.default_rng(seed)
+    return (rng.standard_normal(shape).astype(np.float32),
+            [rng.standard_normal((n, R)).astype(np.float32) for n in shape])
+
+
+# rows across every tile height (32..128) and remainder, runs of 1 to 300
+# columns, inner modes too short to be the run, ranks across the column tiles
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("shape,R", [
+    ((131, 7, 259), 33), ((64, 1, 64), 8), ((1, 1, 1), 1), ((16, 16, 16), 65), ((33, 48, 2), 16),
+    ((97, 129), 100), ((5, 300, 3), 24), ((65, 3, 2, 130), 17), ((2, 3, 4, 5, 6, 7), 9),
+    ((1000, 4, 3), 48), ((12, 20, 31, 8), 130)])
+def test_mttkrp_fp32(shape, R, offset):
+    import torch
+    X, fs = draw(shape, R)
+    ctx = tb.Context()
+    dX, dfs = device(X, offset), [device(f, offset) for f in fs]
+    for mode in range(len(shape)):
+        out = torch.empty(shape[mode], R, device="cuda")
+        torch.cuda.synchronize()
+        tb.mttkrp_dev(dX.data_ptr(), shape, [f.data_ptr() for f in dfs], R, mode, out.data_ptr(),
+                      "fp32", ctx=ctx)
+        ctx.synchronize()
+        assert rel(out.cpu().numpy(), mttkrp64(X, fs, mode)) <= 1e-5, mode
+
+
+def test_mttkrp_fp32_nonfinite_rows():
+    """A NaN or infinity reaches its own output row and no other."""
+    X, fs = draw((40, 37, 29), 20)
+    X[3, 5, 7], X[11, 13, 17] = np.nan, np.inf
+    for mode in range(3):
+        bad = np.zeros(X.shape[mode], bool)
+        bad[[(3, 5, 7)[mode], (11, 13, 17)[mode]]] = True
+        got = tb.mttkrp(X, fs, mode, precision="fp32")
+        assert not np.isfinite(got[bad]).any() and np.isfinite(got[~bad]).all()
+        ok = mttkrp64(np.where(np.isfinite(X), X, 0), fs, mode)
+        assert rel(got[~bad], ok[~bad]) <= 1e-5
+
+
+# both sides of the rank where a single BF16x3 call stops running in FP32,
+# three modes with odd sizes, four modes with runs that suit the tensor-core
+# kernel and with short ones, and two modes
+@pytest.mark.parametrize("shape", [(61, 43, 27), (20, 24, 16, 64), (19, 13, 11, 9), (70, 45)])
+@pytest.mark.parametrize("R", [5, 48, 49, 128, 129])
+def test_bf16x3_route(shape, R):
+    X, fs = draw(shape, R)
+    for mode in range(len(shape)):
+        got = tb.mttkrp(X, fs, mode, precision="bf16x3")
+        assert rel(got, mttkrp64(X, fs, mode)) <= 1e-4, mode
+
+
+@pytest.mark.parametrize("shape,R", [((129, 5, 67), 25), ((3, 4, 300), 65), ((17, 2, 9, 33), 8),
+                                     ((200, 130), 24), ((1, 7, 1), 3)])
+def test_mttkrp_f64(shape, R):
+    rng = np.random.default_rng(3)
+    X = rng.standard_normal(shape)
+    fs = [rng.standard_normal((n, R)) for n in shape]
+    for mode in range(len(shape)):
+        assert rel(tb.mttkrp_f64(X, fs, mode), mttkrp64(X, fs, mode)) <= 1e-12, mode
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("shape,J", [((130, 66, 33), 65), ((4, 128, 64), 64), ((7, 31, 1), 130),
+                                     ((1, 33, 257), 3), ((70000, 2, 3), 2)])
+def test_matrix_product(shape, J, offset):
+    import torch
+    rng = np.random.default_rng(J)
+    X = rng.standard_normal(shape).astype(np.float32)
+    ctx, lib = tb.Context(), _lib.load()
+    dX = device(X, offset)
+    for mode in range(3):
+        M = rng.standard_normal((J, shape[mode])).astype(np.float32)
+        dM = device(M, offset)
+        oshape = shape[:mode] + (J,) + shape[mode + 1:]
+        out = torch.empty(oshape, device="cuda")
+        torch.cuda.synchronize()
+        rc = lib.tsr_nmode_product_dev_f32(ctx.handle, dX.data_ptr(), 3, (C.c_int64 * 3)(*shape),
+                                           dM.data_ptr(), J, shape[mode], mode, out.data_ptr())
+        assert rc == 0
+        ctx.synchronize()
+        ref = np.moveaxis(np.tensordot(M.astype(np.float64), X, (1, mode)), 0, mode)
+        assert rel(out.cpu().numpy(), ref) <= 1e-5, mode
+
+
+# two passes (both sides at least R wide) and one pass per mode (the others)
+@pytest.mark.parametrize("shape,R", [((65, 7, 33), 24), ((9, 8, 7, 6), 33), ((3, 4, 2, 5, 3), 6),
+                                     ((4, 30, 20), 5), ((130, 3, 2), 7), ((40, 50), 8)])
+@pytest.mark.parametrize("precision", ["fp32", "bf16x3"])
+def test_reconstruction_grad(shape, R, precision):
+    import torch
+    G, fs = draw(shape, R)
+    w = np.random.default_rng(1).random(R).astype(np.float32) + 0.5
+    ctx = tb.Context()
+    dG, dw, dfs = device(G, 1), device(w), [device(f) for f in fs]
+    outs = [torch.empty_like(f) for f in dfs]
+    torch.cuda.synchronize()
+    tb.reconstruction_grad_dev(dG.data_ptr(), shape, [f.data_ptr() for f in dfs], R,
+                               [o.data_ptr() for o in outs], dw.data_ptr(), precision, ctx=ctx)
+    ctx.synchronize()
+    for mode, o in enumerate(outs):
+        bound = 1e-5 if precision == "fp32" else 1e-4
+        assert rel(o.cpu().numpy(), mttkrp64(G, fs, mode) * w) <= bound, mode
+
+
+@pytest.mark.parametrize("shape,R", [((129, 3, 43), 33), ((128, 128), 32), ((257, 1, 2), 66),
+                                     ((1, 127, 3), 1), ((5, 26, 4, 65), 24)])
+def test_reconstruct_tiles(shape, R):
+    _, fs = draw(shape, R)
+    ref = (fs[0].astype(np.float64) @ _kr(fs[1:]).T).reshape(shape)
+    assert rel(tb.cp_reconstruct(fs), ref) <= 1e-6
+
+
+def _kr(fs):
+    out = fs[0].astype(np.float64)
+    for f in fs[1:]:
+        out = (out[:, None, :] * f[None]).reshape(-1, out.shape[1])
+    return out
