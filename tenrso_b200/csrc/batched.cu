@@ -68,6 +68,7 @@ struct BatchArgs {
   int* counter;
   int sweeps;
   int stage_off;     // bytes into the dynamic shared memory (0: no room, see add_rows)
+  int ring_off;      // the same, see stream_rows
   double tol;
   float ridge_eps;   // f32 epsilon * R * 10 is formed per instance
 };
@@ -227,6 +228,75 @@ __device__ __forceinline__ float acc_at(const uint64_t (&acc)[4][2 * RQ], int p,
   return __uint_as_float((uint32_t)((r & 1) ? v >> 32 : v));
 }
 
+// acc += sum over q of x_q W[q], q = j0, j0 + split, .. below n, x_q the float4
+// at xp + q * stride. With `ring` (kRing float4s of shared memory per thread,
+// NT apart; its own slots, so no barrier) the loads run kRing - 2 ahead by
+// cp.async; without it four at a time through registers, all of them consumed
+// before the next four start, so a warp waits out a load latency per four rows.
+// Sums and order are the same. 512 instances of 16..96 on 512 threads, 9.0 ms
+// through registers, 7.7 through the ring; fewer than 24 rows per item do not
+// pay for the ring's start (300 instances of 8..40: 0.60 ms against 0.64).
+constexpr int kRing = 8;
+template <int NT, int RQ>
+__device__ __forceinline__ void stream_rows(uint64_t (&acc)[4][2 * RQ], const float4* xp,
+                                            size_t stride, int j0, int n, int split,
+                                            const float* W, uint32_t ring) {
+  constexpr int Rp = 4 * RQ;
+  if (!ring || n < 24 * split) {
+    int j = j0;
+    for (; j + 3 * split < n; j += 4 * split) {
+      float4 xs[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(j + u * split) * stride);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], W + (j + u * split) * Rp);
+    }
+    for (; j < n; j += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)j * stride), W + j * Rp);
+    return;
+  }
+  const int count = j0 < n ? (n - j0 + split - 1) / split : 0;
+  const int pairs = count / 2;
+  const float4* src = xp + (size_t)j0 * stride;
+  const float* w = W + j0 * Rp;
+  const size_t step = (size_t)split * stride;
+  int next = 0;  // first pair not yet requested
+  auto request = [&]() {
+    if (next < pairs) {
+      const uint32_t at = ring + (uint32_t)(next % (kRing / 2)) * (2 * NT * 16);
+      asm volatile(
+          "cp.async.cg.shared.global [%0], [%1], 16;\n\t"
+          "cp.async.cg.shared.global [%2], [%3], 16;" ::"r"(at),
+          "l"(src), "r"(at + NT * 16), "l"(src + step)
+          : "memory");
+      src += 2 * step;
+    }
+    ++next;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int u = 0; u < kRing / 2 - 1; ++u) request();
+  for (int q = 0; q < pairs; ++q) {
+    // the slots requested here held the pair of the previous turn, whose FMAs
+    // have their values
+    request();
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRing / 2 - 1) : "memory");
+    const uint32_t at = ring + (uint32_t)(q % (kRing / 2)) * (2 * NT * 16);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float4 x;
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w)
+                   : "r"(at + u * (NT * 16))
+                   : "memory");
+      fma_row4<RQ>(acc, x, w);
+      w += split * Rp;
+    }
+  }
+  if (count & 1) fma_row4<RQ>(acc, __ldg(src), w);
+  // nothing in flight into the ring when its next use begins
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 // Adds the items' contributions to their rows of M: v[r] of item t0 + thread
 // belongs to row (t / nkq) % rows. All threads of the CTA call it for the same
 // t0. With `stage` (Rp rows of NT + 1 floats of shared memory) the items meet
@@ -281,7 +351,7 @@ __device__ __forceinline__ void transpose_c(const InstSmem& s, int n2p, int Rp, 
 // pass 1: M[i, r] += sum_k (sum_j X[i, j, k] B[j, r]) C[k, r]
 template <int NT, int RQ>
 __device__ void pass_v(const float4* __restrict__ X4, int n0, int n1, int nkq, const float* B,
-                       const float* Ct, float* M, int R, float* stage) {
+                       const float* Ct, float* M, int R, float* stage, uint32_t ring) {
   constexpr int Rp = 4 * RQ;
   const int nq = n0 * nkq;
   const int split = nq >= NT ? 1 : min(n1, NT / nq);
@@ -299,17 +369,7 @@ __device__ void pass_v(const float4* __restrict__ X4, int n0, int n1, int nkq, c
       for (int p = 0; p < 4; ++p)
 #pragma unroll
         for (int r = 0; r < 2 * RQ; ++r) acc[p][r] = 0;
-      const float4* xp = X4 + (size_t)i * n1 * nkq + kq;
-      // four loads of X in flight per thread, then their FMAs in j order
-      int j = g;
-      for (; j + 3 * split < n1; j += 4 * split) {
-        float4 xs[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(j + u * split) * nkq);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], B + (j + u * split) * Rp);
-      }
-      for (; j < n1; j += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)j * nkq), B + j * Rp);
+      stream_rows<NT, RQ>(acc, X4 + (size_t)i * n1 * nkq + kq, nkq, g, n1, split, B, ring);
       // C rows 4kq .. 4kq+3 at column r: one float4 of Ct (lanes read
       // consecutive float4s; the rows of C would all map to one bank)
       const float4* Ct4 = reinterpret_cast<const float4*>(Ct);
@@ -330,7 +390,8 @@ __device__ void pass_v(const float4* __restrict__ X4, int n0, int n1, int nkq, c
 // M[j, r] += sum_k U[j, k, r] C[k, r]
 template <int NT, int RQ>
 __device__ void pass_u(const float4* __restrict__ X4, int n0, int n1, int nkq, const float* A,
-                       const float* Ct, float* M, float* U, int R, float* stage) {
+                       const float* Ct, float* M, float* U, int R, float* stage,
+                       uint32_t ring) {
   constexpr int Rp = 4 * RQ;
   const int nq = n1 * nkq;
   const int split = nq >= NT ? 1 : min(n0, NT / nq);
@@ -348,17 +409,7 @@ __device__ void pass_u(const float4* __restrict__ X4, int n0, int n1, int nkq, c
       for (int p = 0; p < 4; ++p)
 #pragma unroll
         for (int r = 0; r < 2 * RQ; ++r) acc[p][r] = 0;
-      const float4* xp = X4 + (size_t)j * nkq + kq;
-      const size_t istride = (size_t)n1 * nkq;
-      int i = g;
-      for (; i + 3 * split < n0; i += 4 * split) {
-        float4 xs[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) xs[u] = __ldg(xp + (size_t)(i + u * split) * istride);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) fma_row4<RQ>(acc, xs[u], A + (i + u * split) * Rp);
-      }
-      for (; i < n0; i += split) fma_row4<RQ>(acc, __ldg(xp + (size_t)i * istride), A + i * Rp);
+      stream_rows<NT, RQ>(acc, X4 + (size_t)j * nkq + kq, (size_t)n1 * nkq, g, n0, split, A, ring);
       const float4* Ct4 = reinterpret_cast<const float4*>(Ct);
 #pragma unroll
       for (int r = 0; r < Rp; ++r) {
@@ -398,6 +449,8 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
   float* F = a.F + in.f_off;
   float* U = a.uscratch + (size_t)blockIdx.x * a.uscratch_floats;
   float* stage = a.stage_off ? reinterpret_cast<float*>(smem_raw + a.stage_off) : nullptr;
+  const uint32_t ring =
+      a.ring_off ? (uint32_t)__cvta_generic_to_shared(smem_raw + a.ring_off) + threadIdx.x * 16 : 0;
   __shared__ BatchState st;
   __shared__ int ridge_used;
   if (threadIdx.x == 0) {
@@ -429,7 +482,7 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
     // ---- mode 0
     for (int e = threadIdx.x; e < n0 * Rp; e += NT) s.M[e] = 0.f;
     __syncthreads();
-    pass_v<NT, RQ>(X4, n0, n1, nkq, s.B, s.Ct, s.M, R, stage);
+    pass_v<NT, RQ>(X4, n0, n1, nkq, s.B, s.Ct, s.M, R, stage, ring);
     __syncthreads();
     bool ok = solve_mode<NT>(s, s.M, n0, R, Rp, s.GB, s.GC, s.A, s.GA, ridge_eps, &ridge_used);
     // ---- mode 1
@@ -442,7 +495,7 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
         for (int e = threadIdx.x; e < n4; e += NT) u4[e] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
       __syncthreads();
-      pass_u<NT, RQ>(X4, n0, n1, nkq, s.A, s.Ct, s.M, U, R, stage);
+      pass_u<NT, RQ>(X4, n0, n1, nkq, s.A, s.Ct, s.M, U, R, stage, ring);
       __syncthreads();
       ok = solve_mode<NT>(s, s.M, n1, R, Rp, s.GA, s.GC, s.B, s.GB, ridge_eps, &ridge_used);
     }
@@ -454,7 +507,7 @@ __device__ void run_instance(const BatchArgs& a, int id, unsigned char* smem_raw
         const int k = e / RQ, rq = e - k * RQ;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (k < n2) {
-#pragma unroll 4
+#pragma unroll 8
           for (int j = 0; j < n1; ++j) {
             const float4 u = U4[((size_t)j * n2p + k) * RQ + rq];
             const float4 b = B4[j * RQ + rq];
@@ -623,9 +676,10 @@ namespace {
 // all): one 512-thread CTA per SM, or two of 256. A sweep of an instance of
 // w = n0 n1 n2p (rank padded to 4) takes about 20 us (the solves) + 24 us per
 // 1e6 of w on 512 threads, + 33 us on 256; two CTAs on an SM slow each other's
-// passes by a third. The makespan is that of the largest instance or of the
-// whole batch spread over the slots. Measured: 512 instances of 16..96, 8.9 ms
-// (512 x 1) against 12.1; 300 instances of 8..40, 0.89 against 0.57.
+// passes by a third (rates from before the load ring of stream_rows, which took
+// a fifth off each). The makespan is that of the largest instance or of the
+// whole batch spread over the slots. Measured: 512 instances of 16..96, 7.6 ms
+// (512 x 1) against 9.2; 300 instances of 8..40, 0.91 against 0.61.
 void initial_config(const tsr_ctx* ctx, const std::vector<BatchInst>& inst, int* threads,
                     int* ctas_per_sm) {
   double wmax = 0.0, wsum = 0.0;
@@ -736,7 +790,12 @@ int enqueue_run(tsr_ctx* ctx, tsr_batch* bt, int max_iters, double tol, float* d
     const size_t stage = sizeof(float) * 16 * (bt->threads + 1);
     const bool room = bt->smem + stage <= kBatchMaxSmem;
     a.stage_off = room ? (int)bt->smem : 0;
-    const size_t smem = bt->smem + (room ? stage : 0);
+    size_t smem = bt->smem + (room ? stage : 0);
+    // the load ring, 16-byte slots, as long as every CTA of an SM keeps one
+    const size_t at = (smem + 15) / 16 * 16, ring = (size_t)16 * kRing * bt->threads;
+    const size_t most = std::min(kBatchMaxSmem, (size_t)220 * 1024 / std::max(1, bt->ctas_per_sm));
+    a.ring_off = room && at + ring <= most ? (int)at : 0;
+    if (a.ring_off) smem = at + ring;
     switch (bt->threads) {
       case 128: batched_als_kernel<128><<<ctas, 128, smem, ctx->stream>>>(a); break;
       case 512: batched_als_kernel<512><<<ctas, 512, smem, ctx->stream>>>(a); break;
