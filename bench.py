@@ -476,7 +476,7 @@ def run_adjoint(tb, torch, ctx, stream, args, world, dist, rank):
     fptr = [f.data_ptr() for f in dF]
     gptr = [g.data_ptr() for g in dGr]
     steps = max(5, args.steps)
-    # algorithmic bytes: fp32, two MTTKRP passes (X and its transposed copy,
+    # algorithmic bytes: fp32, two passes over X (T and P, in place,
     # 2 x 4 B per element); bf16x3, one two-sided read of X's
     # bf16 halves (4 B per element)
     out = {"workload": "CP loss+gradient 128x96x64x48, rank 32, reg 1e-3",
