@@ -59,7 +59,13 @@ __global__ void __launch_bounds__(4 * BN) mttkrp_f64_kernel(const __grid_constan
   extern __shared__ __align__(16) double sm64[];
   double* As = sm64;                          // [2][F64_BM][F64_P]
   double* Bs = sm64 + 2 * F64_BM * F64_P;     // [2][F64_K][BN]
-  if (g.done && *g.done) return;
+  if (g.done) {
+    // the inverse on the other stream may be setting the flag right now: one
+    // thread looks, so that the CTA stays or leaves as a whole (a CTA that
+    // stays only writes M, which the solve, after the join, then ignores)
+    const int stop = threadIdx.x == 0 ? *(volatile const int*)g.done : 0;
+    if (__syncthreads_or(stop)) return;
+  }
   const ViewArgs& v = g.v;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int tx = tid % TX, ty = tid / TX;

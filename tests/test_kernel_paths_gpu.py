@@ -68,3 +68,24 @@ def test_batched_row_sums(orc, threads, cps, long):
         assert r.iters == info["iters"]
         assert abs(r.fit - info["fit"]) <= 1e-4, (s, R)
     b.close()
+
+
+# the stop decision is taken beside the next sweep's first MTTKRP, and the host
+# looks at it every eighth sweep: stops at sweeps 3, 20, 33, 8 and 13
+@pytest.mark.parametrize("shape,R,tol", [((70, 40, 33), 5, 2e-2), ((70, 40, 33), 5, 3e-3),
+                                         ((70, 40, 33), 5, 3e-4), ((20, 16, 12, 9), 4, 1e-2),
+                                         ((20, 16, 12, 9), 4, 3e-3)])
+def test_cp_als_f64_stops(orc, shape, R, tol):
+    """The sweeps enqueued past a stop leave factors, fit and history as they
+    are. FP64 on both sides: factors to 1e-6, the history to 1e-9, as in the
+    other FP64 CP-ALS tests."""
+    from tenrso_b200 import synth
+    X, _ = synth.dense_lowrank(shape, R, seed=0xF6, dist="uniform", noise=0.01,
+                               dtype=np.float64)
+    init = [synth.uniform(0xF6, 200 + m, (n, R)) for m, n in enumerate(shape)]
+    res = tb.cp_als_f64(X, R, 60, tol, init=init)
+    U, info = orc.cp_als(X, R, 60, tol, init)
+    assert res.iters == info["iters"] and res.convergence.reason == info["reason"]
+    assert np.abs(res.convergence.fit_history - info["fit_history"]).max() <= 1e-9
+    for a, b in zip(res.factors, U):
+        assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
