@@ -514,6 +514,36 @@ int contract_sides(tsr_ctx* ctx, const float* dX, int N, const int64_t* shape,
   return TSR_OK;
 }
 
+// Microseconds of the longest block of the contraction of T and P: each row of
+// each mode is one block, whose threads walk the other indices of its side,
+// about 0.25 us per step of the 256 threads. A short mode beside a long one has
+// few blocks of very many steps.
+double contract_estimate_us(int N, const int64_t* shape, int R) {
+  const int64_t A = prod_range(shape, 0, N - 2), C = shape[N - 2] * shape[N - 1];
+  double steps = 0.0;
+  for (int m = 0; m < N; ++m)
+    if (m >= N - 2 || N > 3)  // (a side of one mode is its own result)
+      steps = std::max(steps, (double)((m < N - 2 ? A : C) / shape[m]) * R / 256.0);
+  return 0.25 * steps;
+}
+
+// Whether T and P (two passes over X, both no larger than X) and their
+// contraction pay against one FP32 pass per mode with its launches and gaps
+// (16 us, so that near-ties stay with two passes). Measured, us, per mode / two passes:
+// 100 x 2 x 200000 rank 32 1945 / 11709, 30 x 30 x 4000 rank 16 64 / 101,
+// 40 x 3000 x 2 x 2 x 40 rank 16 1340 / 5016; and the other way 128^3 rank 32
+// 59 / 50, 100 x 2 x 20000 rank 4 145 / 113, 64 x 64 x 2 x 20000 rank 64
+// 17523 / 3849, 10^6 rank 16 163 / 97, 3000 x 2 x 2 x 2 x 40 x 40 rank 32
+// 7552 / 1584.
+bool sides_pay(int N, const int64_t* shape, int R) {
+  const int64_t A = prod_range(shape, 0, N - 2), C = shape[N - 2] * shape[N - 1];
+  if (A < R || C < R) return false;
+  double passes = 16.0 * (N - 2);
+  for (int m = 0; m < N; ++m) passes += view_estimate_us(shape[m], A * C / shape[m], R);
+  passes -= view_estimate_us(A, C, R) + view_estimate_us(C, A, R);
+  return contract_estimate_us(N, shape, R) <= passes;
+}
+
 // The four loss scalars and the status word in one read-back into pinned
 // memory and one synchronization.
 int read_scalars(tsr_ctx* ctx, const double* d_scalars, double (&sc)[4]) {
@@ -607,14 +637,14 @@ int reconstruction_grad_device(tsr_ctx* ctx, const float* dG, int ndim, const in
                                const FactorTable& ft, int R, const float* dw, int precision,
                                float* const* d_out) {
   // Three or more modes: two FP32 passes over G (T and P) and a small
-  // contraction of each instead of one pass per mode, as long as T and P are
-  // no larger than G. 121x95x63x47 rank 24: 4 FP32 passes 390 us, this 190. A
-  // BF16x3 request takes it too: G comes new with every call, so each of its N
-  // passes would first write a bf16 unfolding.
+  // contraction of each instead of one pass per mode, where that pays.
+  // 121x95x63x47 rank 24: 4 FP32 passes 390 us, this 190. A BF16x3 request
+  // takes it too: G comes new with every call, so each of its N passes would
+  // first write a bf16 unfolding.
   const int64_t total = numel(ndim, shape);
   if (ndim >= 3 && R >= 1 && R <= 256 && total > 0) {
     const int64_t A = prod_range(shape, 0, ndim - 2), C = shape[ndim - 2] * shape[ndim - 1];
-    if (A >= R && C >= R && A <= ((int64_t)1 << 30) && C < INT32_MAX) {
+    if (sides_pay(ndim, shape, R) && A <= ((int64_t)1 << 30) && C < INT32_MAX) {
       void* tp;
       TSR_TRY(slot_get(ctx, SLOT_MISC1, sizeof(float) * (A + C) * R, &tp));
       float *T = (float*)tp, *P = T + A * R;
@@ -643,11 +673,13 @@ int reconstruction_grad_device(tsr_ctx* ctx, const float* dG, int ndim, const in
       TSR_CUDA(cudaMemsetAsync(d_out[n], 0, sizeof(float) * shape[n] * R, ctx->stream));
       continue;
     }
+    // the precision a single MTTKRP of G would run in
+    const int prec = mttkrp_precision(ctx, ndim, shape, n, R, precision);
     ModeOperand op;
-    TSR_TRY(prepare_mode(ctx, dG, ndim, shape, n, precision, 0, &op));
+    TSR_TRY(prepare_mode(ctx, dG, ndim, shape, n, prec, 0, &op));
     float* partials;
     int splits;
-    TSR_TRY(run_mttkrp_partials(ctx, op, ft, R, precision, &partials, &splits));
+    TSR_TRY(run_mttkrp_partials(ctx, op, ft, R, prec, &partials, &splits));
     TSR_TRY(launch_mttkrp_reduce_scaled(ctx, partials, splits, shape[n], R, dw, d_out[n]));
   }
   return TSR_OK;

@@ -126,6 +126,13 @@ int tile_map(const ViewArgs& g) {
 
 }  // namespace
 
+double view_estimate_us(int64_t rows, int64_t cols, int R) {
+  int bn = 0, bm = 0;
+  choose_tile(rows, R, &bn, &bm);
+  const double tile = (double)(bm + 16) * (bn + 8);
+  return 2.0 * (double)(ceil_div(rows, bm) * ceil_div(R, bn)) * tile * (double)cols / 33e6;
+}
+
 void init_view_attributes() {
   for (int i = 0; i < 5; ++i) {
     g_ctas[0][i] = view_ctas_per_sm<16>(kRows[i]);

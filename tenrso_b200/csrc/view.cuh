@@ -64,6 +64,10 @@ void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* i
 // the plan leaves to other kernels.
 ViewPlan plan_view(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
                    int reserve);
+// Microseconds of an MTTKRP of a rows x cols unfolding: its padded FMAs (a tile
+// is at least 32 rows and 16 columns, and costs its fixed part) at the measured
+// rate. Good to about a third.
+double view_estimate_us(int64_t rows, int64_t cols, int R);
 // Partial sums [splits][I_mode][R] (f: one factor per mode; f[mode] unused).
 int launch_view(tsr_ctx* ctx, cudaStream_t s, const float* X, int ndim, const int64_t* shape,
                 int mode, const float* const* f, int R, const ViewPlan& plan, float* partials);

@@ -157,3 +157,30 @@ def _kr(fs):
     for f in fs[1:]:
         out = (out[:, None, :] * f[None]).reshape(-1, out.shape[1])
     return out
+
+
+# both sides of the rule: a short mode beside a long one leaves the contraction
+# of the two passes few blocks of many steps, so those run one pass (two
+# launches) per mode; the others at most five launches in all
+@pytest.mark.parametrize("shape,R,per_mode", [((60, 2, 3000), 16, True),
+                                              ((60, 3000, 2), 16, True),
+                                              ((6, 1200, 2, 2, 6), 16, True),
+                                              ((60, 2, 300), 16, False),
+                                              ((64, 30, 47), 24, False),
+                                              ((6, 12, 2, 2, 16), 16, False)])
+@pytest.mark.parametrize("precision", ["fp32", "bf16x3"])
+def test_reconstruction_grad_route(shape, R, per_mode, precision):
+    import torch
+    G, fs = draw(shape, R)
+    ctx = tb.Context()
+    dG, dfs = device(G), [device(f) for f in fs]
+    outs = [torch.empty_like(f) for f in dfs]
+    torch.cuda.synchronize()
+    before = ctx.launches
+    tb.reconstruction_grad_dev(dG.data_ptr(), shape, [f.data_ptr() for f in dfs], R,
+                               [o.data_ptr() for o in outs], None, precision, ctx=ctx)
+    ctx.synchronize()
+    launches = ctx.launches - before
+    assert launches == 2 * len(shape) if per_mode else launches <= 5
+    for mode, o in enumerate(outs):
+        assert rel(o.cpu().numpy(), mttkrp64(G, fs, mode)) <= 1e-5, mode
