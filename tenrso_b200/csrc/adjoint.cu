@@ -544,6 +544,27 @@ bool sides_pay(int N, const int64_t* shape, int R) {
   return contract_estimate_us(N, shape, R) <= passes;
 }
 
+// The same choice for a prepared BF16x3 tensor without a copy in X's own
+// layout, whose alternative is one tensor-core pass over each mode's bf16
+// unfolding: about 25 us, the 4 bytes per element, and the Khatri-Rao rows (0.2
+// ns per column, 0.8 from four modes on). T and P go through memory three times
+// and may not take much more of it than X. Measured, us, tensor cores / two
+// passes: 301 x 223 x 187 rank 32 156 / 126, 401 x 399 x 397 rank 16 302 / 257,
+// 97 x 83 x 61 x 45 rank 32 1000 / 186; and 401 x 399 x 397 rank 32 327 / 384,
+// 501 x 499 x 497 rank 8 400 / 479, 33 x 41 x 20001 rank 32 365 / 718,
+// 5 x 3001 x 1001 rank 32 649 / 772.
+bool sides_pay_prepared(int N, const int64_t* shape, int R) {
+  const int64_t A = prod_range(shape, 0, N - 2), C = shape[N - 2] * shape[N - 1];
+  const int64_t n = A * C;
+  if ((A + C) * R > std::max<int64_t>(2 * n, (int64_t)1 << 26)) return false;
+  const double two = view_estimate_us(A, C, R) + view_estimate_us(C, A, R) +
+                     contract_estimate_us(N, shape, R) + 12.0 * (double)((A + C) * R) / 6.4e6;
+  double tc = 0.0;
+  for (int m = 0; m < N; ++m)
+    tc += 25.0 + (double)(n / shape[m]) * (N == 3 ? 0.2e-3 : 0.8e-3) + 0.62e-6 * (double)n;
+  return 1.1 * two <= tc;
+}
+
 // The four loss scalars and the status word in one read-back into pinned
 // memory and one synchronization.
 int read_scalars(tsr_ctx* ctx, const double* d_scalars, double (&sc)[4]) {
@@ -910,8 +931,8 @@ int tsr_dense_create_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim, cons
     d->d3.hi = (const __nv_bfloat16*)hp;
     d->d3.lo = (const __nv_bfloat16*)lp;
   }
-  // (a BF16x3 tensor whose view does not suit the two-sided kernel too: two
-  // FP32 passes against one tensor-core pass per mode)
+  // (a BF16x3 tensor whose view does not suit the two-sided kernel too, see
+  // sides_pay_prepared)
   if (!d->d3_on && ndim >= 3 && vshape[0] <= ((int64_t)1 << 30) &&
       vshape[1] * vshape[2] < INT32_MAX) {
     const int64_t v2[2] = {vshape[0], vshape[1] * vshape[2]};
@@ -1077,7 +1098,8 @@ int tsr_cp_loss_grad_dev_f32(tsr_ctx* ctx, const tsr_dense* X, const float* cons
     TSR_TRY(launch_twosided(ctx, ctx->stream, ts));
     return contract_grad(ts.T, ts.P);
   }
-  if (X->v2_on && R <= 32) {
+  if (X->v2_on && R <= 32 &&
+      (X->precision == TSR_PREC_FP32 || sides_pay_prepared(N, X->shape, R))) {
     // FP32: T = X KR(trailing two) and P = X^T KR(leading), both read from X
     // in place: two passes over X's bytes instead of one per mode, and half
     // the FLOPs of N MTTKRPs

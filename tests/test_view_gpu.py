@@ -184,3 +184,31 @@ def test_reconstruction_grad_route(shape, R, per_mode, precision):
     assert launches == 2 * len(shape) if per_mode else launches <= 5
     for mode, o in enumerate(outs):
         assert rel(o.cpu().numpy(), mttkrp64(G, fs, mode)) <= 1e-5, mode
+
+
+# a prepared BF16x3 tensor whose view suits no copy: two FP32 passes (at most
+# six launches) where they pay, else one tensor-core pass and one gradient
+# kernel per mode
+@pytest.mark.parametrize("shape,R,per_mode", [((11, 21, 4001), 32, True), ((5, 9, 4001), 32, True),
+                                              ((61, 43, 27), 16, False),
+                                              ((19, 13, 11, 9), 8, False)])
+def test_loss_grad_route(shape, R, per_mode):
+    import torch
+    X, fs = draw(shape, R)
+    ctx = tb.Context()
+    dX, dfs = device(X), [device(f) for f in fs]
+    outs = [torch.empty_like(f) for f in dfs]
+    torch.cuda.synchronize()
+    D = tb.DenseTensor(dX.data_ptr(), shape, "bf16x3", ctx=ctx)
+    before = ctx.launches
+    loss = D.loss_grad_dev([f.data_ptr() for f in dfs], R, 1e-3, [o.data_ptr() for o in outs])
+    launches = ctx.launches - before
+    D.close()
+    assert launches >= 2 + 2 * len(shape) if per_mode else launches <= 6
+    f64 = [f.astype(np.float64) for f in fs]
+    E = (f64[0] @ _kr(fs[1:]).T).reshape(shape) - X
+    assert abs(loss - (E ** 2).sum() - 1e-3 * sum((f ** 2).sum() for f in f64)) <= 1e-4 * loss
+    for mode, o in enumerate(outs):
+        ref = 2 * np.moveaxis(E, mode, 0).reshape(shape[mode], -1) @ _kr(
+            [f for m, f in enumerate(fs) if m != mode]) + 2e-3 * f64[mode]
+        assert rel(o.cpu().numpy(), ref) <= 1e-4, mode
