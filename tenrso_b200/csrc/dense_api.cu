@@ -465,7 +465,7 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
   std::vector<ModeOperand> ops(ndim);
   size_t pmax = 0;
   const bool fused_unfold = !d3 && !sp && max_iters > 0 && precision == TSR_PREC_BF16X3 &&
-                            unfold3_supported(ndim, shape);
+                            unfold3_supported(ndim, shape) && ((uintptr_t)dX & 15) == 0;
   if (d3) {
     Dense3& d = a.d3;
     a.d3_on = 1;

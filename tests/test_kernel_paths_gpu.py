@@ -89,3 +89,49 @@ def test_cp_als_f64_stops(orc, shape, R, tol):
     assert np.abs(res.convergence.fit_history - info["fit_history"]).max() <= 1e-9
     for a, b in zip(res.factors, U):
         assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
+
+
+# BF16x3 CP-ALS off the single-layout path: bf16 unfoldings and the tensor-core
+# kernels on them. One element into its buffer, a tensor of any shape runs so;
+# aligned, long or high-rank three-mode tensors do (all unfoldings in one pass).
+# Run-scaled kernel: run lengths 8..384, padded k-blocks, odd ranks, several
+# runs per CTA, 4-way weights; (129, 70, 31) and (8, 9, 10, 3, 4): the other one.
+@pytest.mark.parametrize("shape,R,offset", [
+    ((130, 5, 192), 5, 1), ((70, 6, 4, 128), 4, 1), ((40, 7, 384), 7, 1), ((300, 64, 64), 16, 1),
+    ((33, 12, 3, 64), 3, 1), ((70, 6, 48), 6, 1), ((16, 12, 8, 48), 8, 1), ((50, 9, 104), 9, 1),
+    ((24, 40, 8), 5, 1), ((129, 70, 31), 20, 1), ((8, 9, 10, 3, 4), 3, 1), ((80, 72, 88), 70, 1),
+    ((128, 1024, 64), 8, 0), ((80, 72, 88), 70, 0), ((90, 33, 20), 17, 0)])
+def test_cp_als_bf16x3_unfoldings(shape, R, offset):
+    """One sweep against FP64. An MTTKRP is good to 1e-5 of its norm (BF16x3
+    keeps 16 bits of each factor of a product, and the errors average), and each
+    solve multiplies the errors so far by at most the condition of its normal
+    equations; ten times that, once per mode."""
+    import torch
+    rng = np.random.default_rng(sum(shape) + R)
+    X = rng.standard_normal(shape).astype(np.float32)
+    init = [rng.standard_normal((n, R)).astype(np.float32) for n in shape]
+    buf = torch.empty(X.size + offset, device="cuda")
+    buf[offset:].copy_(torch.from_numpy(X.ravel()))
+    d_init = torch.from_numpy(np.concatenate([f.ravel() for f in init])).cuda()
+    out = torch.empty_like(d_init)
+    torch.cuda.synchronize()
+    ctx, launches = tb.Context(), {}
+    for precision in ("fp32", "bf16x3"):
+        before = ctx.launches
+        tb.cp_als_dev(buf.data_ptr() + 4 * offset, shape, R, 1, 0.0, d_init.data_ptr(),
+                      out.data_ptr(), precision, ctx=ctx)
+        launches[precision] = ctx.launches - before
+    one_pass = offset == 0 and shape[1] % 8 == 0 and shape[2] % 8 == 0  # with the norm of X
+    assert launches["bf16x3"] - launches["fp32"] == (0 if one_pass else len(shape))
+    got, off, bound = out.cpu().numpy(), 0, 0.0
+    fs = [f.astype(np.float64) for f in init]
+    for m, n in enumerate(shape):
+        rest = [f for q, f in enumerate(fs) if q != m]
+        kr, H = np.ones((1, R)), np.ones((R, R))
+        for f in rest:
+            kr, H = (kr[:, None, :] * f[None]).reshape(-1, R), H * (f.T @ f)
+        fs[m] = np.linalg.solve(H, (unfold(X, m) @ kr).T).T
+        bound = (bound + 1e-4) * np.linalg.cond(H)
+        err = np.linalg.norm(got[off:off + n * R].reshape(n, R) - fs[m]) / np.linalg.norm(fs[m])
+        assert err <= min(bound, 0.1), (m, err, bound)
+        off += n * R
