@@ -169,18 +169,31 @@ static ViewPlan plan_mode_view(const tsr_ctx* ctx, const ModeOperand& op, int R)
   return plan_view(ctx, op.u.ndim, op.shape, op.u.mode, R, op.resident ? ctx->reserve_sms : 0);
 }
 
-// Measured, us per mode with the unfolding (kernel alone), BF16x3 against FP32
-// in place: 301x223x187 rank 32 106-155 (33) against 67-79 (45), rank 128
-// 187-231 (95) against 140-165 (126); 97x83x61x45 rank 32 270-908 (151-366)
-// against 99-123 (73-97), rank 64 (128-246) against (128-161); 128x96x64x48,
-// whose runs suit the run-scaled tensor-core kernel, rank 32 164-1143 (62-114)
-// against 112-140 (86-116), rank 64 167-1173 (65-120) against 185-238
-// (156-215); 40x33x37 any rank (11-27) against (8-10).
+// A BF16x3 call first writes X's bf16 unfolding. That streams for mode 0, whose
+// unfolding is X's own order (whole float4s where its columns are a multiple of
+// 4), and for long rows; then the tensor cores win on large tensors at the ranks
+// where an FP32 tile of 48 or 64 columns is full: 33..64 and above 112, a
+// multiple of 4 (their Khatri-Rao rows load as float4). Four modes need the
+// run-scaled kernel, and its mode 1. us per call, BF16x3 / FP32 in place:
+//   mode 0, three modes: 400^3 rank 48 226 / 282, rank 64 213 / 331, rank 96
+//     710 / 533, rank 128 500 / 632, rank 32 198 / 187; 333 x 300 x 301 rank 64
+//     159 / 196; 3000 x 60 x 130 rank 64 115 / 149; 700 x 100 x 300 rank 50
+//     154 / 121; odd columns, 301 x 63 x 1001, rank 64 142 / 121; below 2^24
+//     elements, 301 x 223 x 187, rank 64 109 / 88;
+//   its other modes: 400^3 rank 64 369 / 332 and 348 / 359;
+//   four modes: 96 x 97 x 80 x 64 rank 48 251 / 186, 163 / 233, 1057 / 220,
+//     297 / 245; 40 x 50 x 100 x 90 (no run-scaled kernel) 390 / 146, 238 / 142,
+//     383 / 137, 201 / 124 at rank 64.
 int mttkrp_precision(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,
                      int precision) {
   if (precision != TSR_PREC_BF16X3 || R > 128) return precision;
-  const bool runs = plan_tc(ctx, make_unfolding(ndim, shape, mode), R).run_length > 0;
-  return R <= 48 || !runs ? TSR_PREC_FP32 : precision;
+  if (R <= 32 || R % 4 != 0 || numel(ndim, shape) < ((int64_t)1 << 24)) return TSR_PREC_FP32;
+  int64_t B = 1;
+  for (int m = mode + 1; m < ndim; ++m) B *= shape[m];
+  const bool streams = ndim <= 3 && mode == 0 && B % 4 == 0 && (R <= 64 || R > 112);
+  const bool runs = ndim >= 4 && mode == 1 && B >= 1024 && R <= 64 &&
+                    plan_tc(ctx, make_unfolding(ndim, shape, mode), R).run_length > 0;
+  return streams || runs ? precision : TSR_PREC_FP32;
 }
 
 size_t mode_partial_floats(const tsr_ctx* ctx, const ModeOperand& op, int R, int precision) {

@@ -212,3 +212,33 @@ def test_loss_grad_route(shape, R, per_mode):
         ref = 2 * np.moveaxis(E, mode, 0).reshape(shape[mode], -1) @ _kr(
             [f for m, f in enumerate(fs) if m != mode]) + 2e-3 * f64[mode]
         assert rel(o.cpu().numpy(), ref) <= 1e-4, mode
+
+
+# where a single BF16x3 call writes a bf16 unfolding and runs the tensor cores
+# (three launches), and where it reads X in FP32 (two): ranks, modes, column
+# counts and tensor sizes on both sides of the rule
+@pytest.mark.parametrize("shape,R,tensor_cores", [
+    ((258, 260, 252), 36, {0}), ((258, 260, 252), 64, {0}), ((258, 260, 252), 116, {0}),
+    ((258, 260, 252), 32, set()), ((258, 260, 252), 50, set()), ((258, 260, 252), 96, set()),
+    ((250, 260, 252), 64, set()), ((261, 259, 251), 64, set()), ((65, 64, 66, 64), 48, {1}),
+    ((65, 64, 66, 64), 68, set()), ((65, 64, 66, 63), 48, set()), ((4100, 4100), 64, {0})])
+def test_bf16x3_large_route(shape, R, tensor_cores):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(5)
+    X = torch.randn(*shape, generator=g, device="cuda")
+    fs = [torch.randn(n, R, generator=g, device="cuda") for n in shape]
+    ctx = tb.Context()
+    for mode in range(len(shape)):
+        out = torch.empty(shape[mode], R, device="cuda")
+        torch.cuda.synchronize()
+        before = ctx.launches
+        tb.mttkrp_dev(X.data_ptr(), shape, [f.data_ptr() for f in fs], R, mode, out.data_ptr(),
+                      "bf16x3", ctx=ctx)
+        assert ctx.launches - before == (3 if mode in tensor_cores else 2), mode
+        kr = torch.ones(1, R, device="cuda", dtype=torch.float64)
+        for m, f in enumerate(fs):
+            if m != mode:
+                kr = (kr[:, None, :] * f.double()[None]).reshape(-1, R)
+        ref = X.double().movedim(mode, 0).reshape(shape[mode], -1) @ kr
+        bound = 1e-4 if mode in tensor_cores else 1e-5
+        assert float((out.double() - ref).norm() / ref.norm()) <= bound, mode
