@@ -59,11 +59,16 @@ void choose_tile(int64_t rows, int R, int* bn, int* bm) {
 // Tile of a product that is not split over its contraction: the least work of
 // the busiest SM (its tiles, each padded by the fixed part of a step), weighted
 // by how well the warps it holds cover latency (w / (w + 4): 8 warps reach two
-// thirds, 16 four fifths of the rate of a full SM).
-void choose_tile_unsplit(const tsr_ctx* ctx, int64_t rows, int64_t R, int64_t batch, int* bn,
-                         int* bm) {
+// thirds, 16 four fifths of the rate of a full SM). A tile that is turned
+// through shared memory on its way out is at most 32 columns wide: then four
+// CTAs share an SM and one's stores overlap another's loads, which short
+// contractions are made of. us at widths 64 / 32: 16 x 1000000 to 64 193 / 156,
+// 64 x 256 x 256 to 64 33 / 31, 256 x 64 x 64 to 256 35 / 31, 30 x 30 x 4000
+// to 64 37 / 29; no size measured wants the wider ones.
+void choose_tile_unsplit(const tsr_ctx* ctx, int64_t rows, int64_t R, int64_t batch, bool turned,
+                         int* bn, int* bm) {
   double best = 0.0;
-  for (int wi = 0; wi < 5; ++wi)
+  for (int wi = 0; wi < (turned ? 3 : 5); ++wi)
     for (int ri = 0; ri < 5; ++ri) {
       const int w = kWidths[wi], m = kRows[ri];
       const int64_t tiles = ceil_div(rows, m) * ceil_div(R, w) * batch;
@@ -231,13 +236,13 @@ int launch_view_matrix(tsr_ctx* ctx, cudaStream_t s, const float* X, int64_t A, 
     g.batch = 1;
   }
   g.map = tile_map(g);
-  constexpr int64_t most = (int64_t)65535 * 64;  // columns of one launch
-  for (int64_t j0 = 0; j0 < J; j0 += most) {
-    g.R = (int)std::min<int64_t>(J - j0, most);
+  for (int64_t j0 = 0, cols; j0 < J; j0 += cols) {
+    int bn, bm;
+    choose_tile_unsplit(ctx, g.rows, J - j0, g.batch, B > 1, &bn, &bm);
+    cols = std::min<int64_t>(J - j0, (int64_t)65535 * bn);  // one launch's column tiles
+    g.R = (int)cols;
     g.inner = mat + j0 * I;
     g.out = Y + j0 * g.out_col;
-    int bn, bm;
-    choose_tile_unsplit(ctx, g.rows, g.R, g.batch, &bn, &bm);
     const dim3 grid((unsigned)ceil_div(g.rows, bm),
                     (unsigned)std::min<int64_t>(g.batch, 65535), (unsigned)ceil_div(g.R, bn));
     TSR_TRY(dispatch(ctx, s, g, bn, bm, grid));

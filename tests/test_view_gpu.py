@@ -242,3 +242,24 @@ def test_bf16x3_large_route(shape, R, tensor_cores):
         ref = X.double().movedim(mode, 0).reshape(shape[mode], -1) @ kr
         bound = 1e-4 if mode in tensor_cores else 1e-5
         assert float((out.double() - ref).norm() / ref.norm()) <= bound, mode
+
+
+# more column tiles than one launch holds, in both output layouts; contractions
+# shorter than a chunk, expanding, with rows on both sides of a tile
+@pytest.mark.parametrize("A,I,B,J", [(1, 2, 3, 65535 * 32 + 17), (2, 2, 1, 65535 * 16 + 17),
+                                     (1, 16, 3001, 64), (301, 5, 5, 301), (3, 1, 130, 33),
+                                     (2, 30, 127, 48), (40, 10, 10, 65)])
+def test_matrix_product_expanding(A, I, B, J):
+    """At most 30 products per entry: the reconstruction's bound."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(J)
+    X = torch.randn(A, I, B, generator=g, device="cuda")
+    M = torch.randn(J, I, generator=g, device="cuda")
+    out = torch.empty(A, J, B, device="cuda")
+    torch.cuda.synchronize()
+    ctx, lib = tb.Context(), _lib.load()
+    assert lib.tsr_nmode_product_dev_f32(ctx.handle, X.data_ptr(), 3, (C.c_int64 * 3)(A, I, B),
+                                         M.data_ptr(), J, I, 1, out.data_ptr()) == 0
+    ctx.synchronize()
+    ref = torch.einsum("ji,aib->ajb", M.double(), X.double())
+    assert float((out.double() - ref).norm() / ref.norm()) <= 1e-6
