@@ -163,13 +163,19 @@ __global__ void __launch_bounds__(256) gram_reduce_kernel(const double* __restri
 // by bisection on Sturm counts, each eigenvector of T from its twisted
 // factorisation (T - lambda I = L D L^T from the top and U D U^T from the
 // bottom, joined at the row with the smallest |gamma|), and the reflections
-// applied back. All FP64. An eigenvector comes out to about eps |T| / gap, so
-// the host takes this path only where the leading eigenvalues are separated by
-// more than 1e-8 of the largest, and the Jacobi solver below otherwise
-// (repeated or zero eigenvalues, non-finite tensors) and beyond kTriRows rows.
-// About 4/3 I^3 operations in three launches for all modes together, against
-// some ten Jacobi sweeps of 6 I^3 in three launches per round each.
+// applied back. All FP64. Each eigenvector comes out by itself, to about eps |T|
+// / gap, so the host takes this path only where the leading eigenvalues are
+// separated by more than kTriGap of the largest, and the Jacobi solver below
+// otherwise (repeated or zero eigenvalues, non-finite tensors) and beyond
+// kTriRows rows. Off-diagonal of U^T U as returned in FP32, largest of eight
+// matrices of 40 rows: 3.3e-8 at gaps of 1.2e-8, 7e-9 at 1.1e-7, 2e-9 at 2e-7,
+// where rounding exact vectors to FP32 alone leaves about 2e-8.
+// About 4/3 I^3 operations in two launches for all modes together, against
+// some ten Jacobi sweeps of 6 I^3 in three launches per round each. 160 rows are
+// what one CTA holds: 50 doubles of the matrix in each of 512 threads, of 128
+// registers at most.
 constexpr int kTriRows = 160;
+constexpr double kTriGap = 1e-7;
 
 struct TriMode {
   const double* G;  // I x I
@@ -971,7 +977,7 @@ int init_factors_device(tsr_ctx* ctx, const float* dX, int ndim, const int64_t* 
       const double* l = h.data() + lam_off[t];
       const int n = (int)std::min<int64_t>(q.k + 1, q.I);
       bool apart = std::isfinite(l[0]) && l[0] > 0.0;
-      for (int i = 0; i + 1 < n; ++i) apart = apart && l[i] - l[i + 1] > 1e-8 * l[0];
+      for (int i = 0; i + 1 < n; ++i) apart = apart && l[i] - l[i + 1] > kTriGap * l[0];
       if (!apart) continue;
       q.ready = true;
       q.V = tri.m[t].U;

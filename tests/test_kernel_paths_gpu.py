@@ -135,3 +135,35 @@ def test_cp_als_bf16x3_unfoldings(shape, R, offset):
         err = np.linalg.norm(got[off:off + n * R].reshape(n, R) - fs[m]) / np.linalg.norm(fs[m])
         assert err <= min(bound, 0.1), (m, err, bound)
         off += n * R
+
+
+# leading eigenvalues 1 + delta r on both sides of the separation that the
+# tridiagonalisation needs (a dozen launches; the Jacobi rotations take hundreds)
+@pytest.mark.parametrize("n", [40, 160])
+@pytest.mark.parametrize("delta,jacobi", [(1.2e-8, True), (5e-8, True), (2e-7, False),
+                                          (1e-5, False)])
+def test_svd_start_close_eigenvalues(n, delta, jacobi):
+    """The eigenvectors are products of two dyadic reflections, scaled by values
+    of few bits, so X is exact in FP32 and its Gram has exactly these
+    eigenvalues. The result is no further from orthonormal than rounding
+    exact vectors to FP32 allows: 2 |u| |2^-25 v| = 6e-8."""
+    rng = np.random.default_rng(n)
+    w = 1 << ((n - 1).bit_length() - 1)
+    Q = np.eye(n)
+    for _ in range(2):
+        v = np.zeros(n)
+        v[rng.permutation(n)[:w]] = 1
+        v *= rng.choice([-1, 1], n)
+        Q = Q @ (np.eye(n) - np.outer(v, v) * 2 / w)
+    s, t = np.ones(n), np.zeros(n)
+    s[9:] = np.round(np.linspace(0.95, 0.1, n - 9) * 256) / 256
+    m, e = np.frexp(np.sqrt(delta * np.arange(9)[::-1]))
+    t[:9] = np.ldexp(np.round(m * 1024) / 1024, e)
+    X = np.concatenate([Q * s, Q * t], 1)
+    assert (X.astype(np.float32) == X).all()
+    ctx = tb.Context()
+    before = ctx.launches
+    F = tb.initialize_factors(X.reshape(n, 2, n), 8, "svd", seed=1, ctx=ctx)
+    assert (ctx.launches - before > 100) == jacobi
+    for V in (F[0].astype(np.float64), F[2].astype(np.float64)):
+        assert np.abs(V.T @ V - np.eye(8)).max() <= 6e-8
