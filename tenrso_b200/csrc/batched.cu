@@ -37,7 +37,16 @@ namespace tsr {
 namespace {
 
 constexpr int kBatchMaxR = 16;
+// Rows of M that so many items (float4s of the last mode) meet in are worth a
+// resident CTA: the staging rows of add_rows against shared-memory atomics. us,
+// two 256-thread CTAs with atomics / one with the staging rows, instances of
+// 102 KB, rank 16, last mode 16: 4095 / 5549, 32: 6976 / 7758, 48: 11033 /
+// 10208, 64: 14465 / 11663, 128: 34477 / 19055.
+constexpr int kCrowded = 12;
 constexpr size_t kBatchMaxSmem = 200 * 1024;
+// Shared memory of an SM, and what a CTA takes of it beside its dynamic part
+// (1 KB, and the kernel's static arrays).
+constexpr size_t kSmSmem = 228 * 1024, kBatchOwnSmem = 1024 + 512;
 
 struct BatchInst {
   int n0, n1, n2, n2p;  // mode sizes; n2p = n2 rounded up to a multiple of 4
@@ -301,8 +310,8 @@ __device__ __forceinline__ void stream_rows(uint64_t (&acc)[4][2 * RQ], const fl
 // belongs to row (t / nkq) % rows. All threads of the CTA call it for the same
 // t0. With `stage` (Rp rows of NT + 1 floats of shared memory) the items meet
 // there and one thread sums each row's run of nkq; without it (instances that
-// fill the shared memory) they add with shared-memory atomics, which a warp's
-// lanes on one row serialise: at 96^3 rank 16 that took most of a pass.
+// leave it no room, see plan_smem) they add with shared-memory atomics, which a
+// warp's lanes on one row serialise: at 96^3 rank 16 that took most of a pass.
 template <int NT, int Rp>
 __device__ __forceinline__ void add_rows(const float (&v)[Rp], int t0, int items, int nkq,
                                          int rows, bool split, int R, float* M, float* stage) {
@@ -648,6 +657,8 @@ struct tsr_batch {
   std::vector<int> order;
   int64_t x_floats = 0, f_floats = 0;
   size_t smem = 0;
+  int rq = 1;   // the largest padded rank, in fours
+  int nkq = 1;  // the longest last mode, in fours
   int64_t uscratch_floats = 0;
   tsr::BatchInst* d_inst = nullptr;
   int* d_order = nullptr;
@@ -672,6 +683,34 @@ struct tsr_batch {
 namespace tsr {
 namespace {
 
+// Dynamic shared memory of a launch: the largest instance, then (where they
+// fit) the staging rows of add_rows and the load ring of stream_rows.
+struct SmemPlan {
+  int held;  // CTAs that one SM holds
+  int stage_off = 0, ring_off = 0;
+  size_t bytes;
+};
+
+SmemPlan plan_smem(const tsr_batch* bt, int threads, int ctas_per_sm) {
+  SmemPlan p;
+  p.bytes = bt->smem;
+  p.held = std::max(
+      1, std::min(std::max(1, ctas_per_sm), (int)(kSmSmem / (bt->smem + kBatchOwnSmem))));
+  auto most = [&]() { return std::min(kBatchMaxSmem, kSmSmem / p.held - kBatchOwnSmem); };
+  const size_t stage = sizeof(float) * 4 * bt->rq * (threads + 1);
+  if (bt->nkq >= kCrowded)
+    while (p.held > 1 && bt->smem + stage > most()) --p.held;
+  if (bt->smem + stage > most()) return p;
+  p.stage_off = (int)bt->smem;
+  p.bytes = bt->smem + stage;
+  const size_t at = (p.bytes + 15) / 16 * 16, ring = (size_t)16 * kRing * threads;
+  if (at + ring <= most()) {  // 16-byte slots; never at the price of a CTA
+    p.ring_off = (int)at;
+    p.bytes = at + ring;
+  }
+  return p;
+}
+
 // The configuration a new batch starts with (tsr_batch_autotune times them
 // all): one 512-thread CTA per SM, or two of 256. A sweep of an instance of
 // w = n0 n1 n2p (rank padded to 4) takes about 20 us (the solves) + 24 us per
@@ -679,20 +718,22 @@ namespace {
 // passes by a third (rates from before the load ring of stream_rows, which took
 // a fifth off each). The makespan is that of the largest instance or of the
 // whole batch spread over the slots. Measured: 512 instances of 16..96, 7.6 ms
-// (512 x 1) against 9.2; 300 instances of 8..40, 0.91 against 0.61.
-void initial_config(const tsr_ctx* ctx, const std::vector<BatchInst>& inst, int* threads,
-                    int* ctas_per_sm) {
+// (512 x 1) against 9.2; 300 instances of 8..40, 0.91 against 0.61. Where the SM
+// holds one CTA of 256 only, it is 512: 296 instances of 4 x 5900 x 8 rank 4,
+// 12.4 ms against 13.5, of 350 x 16 x 350 rank 16, 13.6 against 24.8.
+void initial_config(const tsr_ctx* ctx, const tsr_batch* bt, int* threads, int* ctas_per_sm) {
   double wmax = 0.0, wsum = 0.0;
-  for (const BatchInst& in : inst) {
+  for (const BatchInst& in : bt->inst) {
     const double w = 1e-6 * in.n0 * in.n1 * in.n2p * 4 * in.rq;
     wmax = std::max(wmax, w);
     wsum += w;
   }
-  const double n = (double)inst.size(), sms = ctx->sm_count;
+  const double n = (double)bt->n_inst, sms = ctx->sm_count;
   const double one = std::max(20 + 24 * wmax, (20 * n + 24 * wsum) / sms);
   const double two = std::max(20 + 33 * wmax, (20 * n + 44 * wsum) / (2 * sms));
-  *threads = one <= two ? 512 : 256;
-  *ctas_per_sm = one <= two ? 1 : 2;
+  const bool wide = one <= two || plan_smem(bt, 256, 2).held < 2;
+  *threads = wide ? 512 : 256;
+  *ctas_per_sm = wide ? 1 : 2;
 }
 
 int batch_validate(int n_inst, const int64_t* shapes, const int64_t* ranks) {
@@ -787,15 +828,10 @@ int enqueue_run(tsr_ctx* ctx, tsr_batch* bt, int max_iters, double tol, float* d
     a.sweeps = std::min(S, max_iters - l * S);
     a.tol = tol;
     a.ridge_eps = std::numeric_limits<float>::epsilon() * 10.0f;
-    const size_t stage = sizeof(float) * 16 * (bt->threads + 1);
-    const bool room = bt->smem + stage <= kBatchMaxSmem;
-    a.stage_off = room ? (int)bt->smem : 0;
-    size_t smem = bt->smem + (room ? stage : 0);
-    // the load ring, 16-byte slots, as long as every CTA of an SM keeps one
-    const size_t at = (smem + 15) / 16 * 16, ring = (size_t)16 * kRing * bt->threads;
-    const size_t most = std::min(kBatchMaxSmem, (size_t)220 * 1024 / std::max(1, bt->ctas_per_sm));
-    a.ring_off = room && at + ring <= most ? (int)at : 0;
-    if (a.ring_off) smem = at + ring;
+    const SmemPlan p = plan_smem(bt, bt->threads, bt->ctas_per_sm);
+    a.stage_off = p.stage_off;
+    a.ring_off = p.ring_off;
+    const size_t smem = p.bytes;
     switch (bt->threads) {
       case 128: batched_als_kernel<128><<<ctas, 128, smem, ctx->stream>>>(a); break;
       case 512: batched_als_kernel<512><<<ctas, 512, smem, ctx->stream>>>(a); break;
@@ -921,13 +957,15 @@ int tsr_batch_create_f32(tsr_ctx* ctx, int n_inst, const int64_t* shapes, const 
     bt->x_floats += (int64_t)in.n0 * in.n1 * in.n2p;
     in.f_off = bt->f_floats;
     bt->f_floats += (int64_t)(in.n0 + in.n1 + in.n2) * in.R;
+    bt->rq = std::max(bt->rq, in.rq);
+    bt->nkq = std::max(bt->nkq, in.n2p / 4);
     bt->smem = std::max(bt->smem, inst_smem_bytes(in.n0, in.n1, in.n2p, in.rq));
     bt->uscratch_floats =
         std::max<int64_t>(bt->uscratch_floats, (int64_t)in.n1 * in.n2p * 4 * in.rq);
     work[b] = (double)in.n0 * in.n1 * in.n2p * (4 * in.rq + 4);
   }
   bt->uscratch_floats = (bt->uscratch_floats + 3) / 4 * 4;
-  initial_config(ctx, bt->inst, &bt->threads, &bt->ctas_per_sm);
+  initial_config(ctx, bt, &bt->threads, &bt->ctas_per_sm);
   auto cleanup = [&](int rc) {
     tsr_batch_destroy(bt);
     return rc;

@@ -167,3 +167,43 @@ def test_svd_start_close_eigenvalues(n, delta, jacobi):
     assert (ctx.launches - before > 100) == jacobi
     for V in (F[0].astype(np.float64), F[2].astype(np.float64)):
         assert np.abs(V.T @ V - np.eye(8)).max() <= 6e-8
+
+
+# instances of about 100 KB, where the buffers beside them decide how many CTAs
+# an SM holds: staging rows kept (few columns), given up for the second CTA
+# (short rows), the second CTA given up for them (long rows)
+@pytest.mark.parametrize("shape,R", [((4, 2700, 8), 4), ((4, 3200, 16), 4), ((16, 690, 48), 16),
+                                     ((16, 716, 16), 16), ((9, 1450, 17), 7)])
+@pytest.mark.parametrize("threads,cps", [(128, 4), (256, 2), (512, 1)])
+def test_batched_large_instances(shape, R, threads, cps):
+    """One sweep against FP64: row sums in FP32 to 1e-5, each solve multiplies
+    the errors so far by at most the condition of its normal equations."""
+    rng = np.random.default_rng(sum(shape))
+    X = rng.standard_normal((3,) + shape).astype(np.float32)
+    inits = [[rng.standard_normal((n, R)).astype(np.float32) for n in shape] for _ in range(3)]
+    b = tb.BatchedCpAls(list(X), [R] * 3)
+    b.set_config(threads, 0, cps)
+    for x, init, r in zip(X, inits, b.cp_als(1, 0.0, init=inits)):
+        fs, bound = [f.astype(np.float64) for f in init], 0.0
+        for m, n in enumerate(shape):
+            kr, H = np.ones((1, R)), np.ones((R, R))
+            for q, f in enumerate(fs):
+                if q != m:
+                    kr, H = (kr[:, None, :] * f[None]).reshape(-1, R), H * (f.T @ f)
+            fs[m] = np.linalg.solve(H, (unfold(x, m) @ kr).T).T
+            bound = (bound + 1e-5) * np.linalg.cond(H)
+            err = np.linalg.norm(r.factors[m] - fs[m]) / np.linalg.norm(fs[m])
+            assert err <= min(bound, 0.1), (m, err, bound)
+    b.close()
+
+
+@pytest.mark.parametrize("shape,R,expect", [((4, 5900, 8), 4, (512, 1)),
+                                            ((4, 3200, 16), 4, (256, 2)),
+                                            ((16, 690, 48), 16, (512, 1)),
+                                            ((20, 20, 20), 4, (256, 2))])
+def test_batched_initial_config(shape, R, expect):
+    """Two CTAs per SM only where the SM holds two."""
+    b = tb.BatchedCpAls([np.ones(shape, np.float32)] * 400, [R] * 400)
+    config = b.config
+    b.close()
+    assert (config["threads"], config["ctas_per_sm"]) == expect
