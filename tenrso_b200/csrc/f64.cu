@@ -403,6 +403,31 @@ void init_f64_attributes() {
   cudaFuncSetAttribute(solve_f64_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 }
 
+// Gives a call's larger device copies back when it ends: an FP64 tensor may be
+// most of the GPU, and the context would keep it until it is destroyed. Slots
+// that an earlier call had already grown, and small ones (kept, so that repeated
+// small calls allocate nothing), stay.
+struct ReturnSlots {
+  static constexpr size_t kKeep = (size_t)64 << 20;
+  static constexpr int kSlots[4] = {SLOT_TENSOR, SLOT_FACTORS, SLOT_OUT, SLOT_PARTIALS};
+  tsr_ctx* ctx;
+  size_t before[4];
+  explicit ReturnSlots(tsr_ctx* c) : ctx(c) {
+    for (int i = 0; i < 4; ++i) before[i] = c->slots[kSlots[i]].bytes;
+  }
+  ~ReturnSlots() {
+    for (int i = 0; i < 4; ++i) {
+      Buffer& b = ctx->slots[kSlots[i]];
+      if (b.bytes <= before[i] || b.bytes <= kKeep) continue;
+      cudaStreamSynchronize(ctx->aux);
+      cudaStreamSynchronize(ctx->stream);
+      cudaFree(b.ptr);
+      b.ptr = nullptr;
+      b.bytes = 0;
+    }
+  }
+};
+
 // cp_als<f64> on device data (dX row-major FP64; factors FP64 in d_out).
 int cp_als_f64_device(tsr_ctx* ctx, const double* dX, int ndim, const int64_t* shape,
                       int64_t rank, int max_iters, double tol, double time_limit_s,
@@ -516,6 +541,7 @@ int tsr_mttkrp_f64(tsr_ctx* ctx, const double* tensor, int ndim, const int64_t* 
   TSR_TRY(validate_mttkrp(ndim, shape, n_factors, factor_rows, factor_cols, mode));
   TSR_TRY(check_sizes(ndim, shape, factor_cols[0]));
   TSR_TRY(check_ctx(ctx));
+  const ReturnSlots give_back(ctx);
   const int R = (int)factor_cols[0];
   const int64_t n = numel(ndim, shape);
   int64_t ftotal = 0;
@@ -573,6 +599,7 @@ int tsr_cp_als_f64(tsr_ctx* ctx, const double* tensor, int ndim, const int64_t* 
     }
     init = init_buf.data();
   }
+  const ReturnSlots give_back(ctx);
   void *xp, *fp;
   TSR_TRY(slot_get(ctx, SLOT_TENSOR, sizeof(double) * std::max<int64_t>(n, 1), &xp));
   TSR_TRY(slot_get(ctx, SLOT_FACTORS, sizeof(double) * std::max<int64_t>(ftotal, 1), &fp));

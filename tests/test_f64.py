@@ -75,3 +75,23 @@ def test_cp_als_f64_seeded_random_init_and_validation(orc):
         tb.cp_als_f64(X, 0, 5, 0.0)
     with pytest.raises(tb.TenrsoError, match="Invalid tolerance"):
         tb.cp_als_f64(X, 2, 5, 1.0)
+
+
+def test_f64_calls_give_their_tensor_back():
+    """A call's device copy of a large tensor does not stay with the context."""
+    import torch
+    X = np.zeros((320, 320, 400))
+    X[7, 11, 13] = 2.0
+    fs = [np.ones((n, 2)) * (1 + np.arange(2)) for n in X.shape]
+    ctx = tb.Context()
+    small = [np.ones((n, 2)) for n in (8, 9, 10)]
+    tb.mttkrp_f64(np.ones((8, 9, 10)), small, 0, ctx=ctx)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    got = tb.mttkrp_f64(X, fs, 1, ctx=ctx)
+    assert got[11].tolist() == [2.0, 8.0] and np.count_nonzero(got) == 2
+    assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
+    res = tb.cp_als_f64(X + 1.0, 2, 2, 0.0, seed=1, ctx=ctx)
+    assert np.isfinite(res.fit)
+    assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
+    ctx.close()
