@@ -35,6 +35,7 @@ struct M64Args {
 };
 
 constexpr int kF64Look = 8;
+constexpr int64_t kF64Columns = (int64_t)1 << 31;  // of one launch's unfolding
 constexpr int F64_BM = 64, F64_K = 32, F64_P = F64_K + 1;
 
 template <int BN>
@@ -303,27 +304,25 @@ void go_f64(cudaStream_t s, const M64Args& g, dim3 grid) {
   mttkrp_f64_kernel<BN><<<grid, 4 * BN, f64_smem<BN>(), s>>>(g);
 }
 
-int launch_mttkrp_f64(tsr_ctx* ctx, const double* X, int ndim, const int64_t* shape,
-                      const double* const* U, int R, int mode, double* M,
-                      const int* done = nullptr) {
+// Rows [c0, c0 + len) of mode `cut` of the contraction, added into M.
+int launch_mttkrp_f64_part(tsr_ctx* ctx, const double* X, int ndim, const int64_t* shape,
+                           const double* const* U, int R, int mode, int cut, int64_t c0,
+                           int64_t len, double* M, const int* done) {
   cudaStream_t s = ctx->stream;
   M64Args g;
   std::memset(&g, 0, sizeof(g));
-  int64_t J = 1;
-  for (int m = 0; m < ndim; ++m)
-    if (m != mode) J *= shape[m];
-  TSR_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * shape[mode] * R, s));
-  if (shape[mode] == 0 || R == 0 || J == 0) return TSR_OK;
-  if (J >= (int64_t)UINT32_MAX) return fail(TSR_E_UNSUPPORTED, "unfolding too wide");
+  int64_t st = 1;  // elements between indices of `cut`
+  for (int m = cut + 1; m < ndim; ++m) st *= shape[m];
   int inner;
-  describe_view(ndim, shape, mode, &g.v, &inner);
+  describe_view(ndim, shape, mode, &g.v, &inner, cut, len);
   g.v.R = R;
-  g.X = X;
+  g.X = X + c0 * st;
   g.M = M;
   g.done = done;
-  g.inner = U[inner];
+  auto rows_of = [&](int m) { return U[m] + (m == cut ? c0 * R : 0); };
+  g.inner = rows_of(inner);
   for (int m = 0, p = 0; m < ndim; ++m)
-    if (m != mode && m != inner) g.f[p++] = U[m];
+    if (m != mode && m != inner) g.f[p++] = rows_of(m);
   const int64_t share = ceil_div(R, ceil_div(R, 32));
   const int bn = share <= 8 ? 8 : share <= 16 ? 16 : share <= 24 ? 24 : 32;
   const int64_t tiles = ceil_div(g.v.rows, F64_BM) * ceil_div(R, bn);
@@ -343,6 +342,27 @@ int launch_mttkrp_f64(tsr_ctx* ctx, const double* X, int ndim, const int64_t* sh
   }
   ctx->launches++;
   TSR_CUDA(cudaGetLastError());
+  return TSR_OK;
+}
+
+int launch_mttkrp_f64(tsr_ctx* ctx, const double* X, int ndim, const int64_t* shape,
+                      const double* const* U, int R, int mode, double* M,
+                      const int* done = nullptr) {
+  int64_t J = 1;
+  for (int m = 0; m < ndim; ++m)
+    if (m != mode) J *= shape[m];
+  TSR_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * shape[mode] * R, ctx->stream));
+  if (shape[mode] == 0 || R == 0 || J == 0) return TSR_OK;
+  // The kernel counts runs, chunks and a run's columns in 32 bits: a wider
+  // unfolding is taken in pieces of its longest contracted mode, whose sums meet
+  // in M as the splits do.
+  int cut = mode == 0 ? 1 : 0;
+  for (int m = 0; m < ndim; ++m)
+    if (m != mode && shape[m] > shape[cut]) cut = m;
+  const int64_t part = std::max<int64_t>(1, kF64Columns / (J / shape[cut]));
+  for (int64_t c0 = 0; c0 < shape[cut]; c0 += part)
+    TSR_TRY(launch_mttkrp_f64_part(ctx, X, ndim, shape, U, R, mode, cut, c0,
+                                   std::min(part, shape[cut] - c0), M, done));
   return TSR_OK;
 }
 

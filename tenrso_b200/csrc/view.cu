@@ -83,35 +83,36 @@ void choose_tile_unsplit(const tsr_ctx* ctx, int64_t rows, int64_t R, int64_t ba
     }
 }
 
-// The contraction of one mode: which contracted mode is the inner one and the
-// strides of all of them. The inner mode is the fastest contracted one, where
-// a chunk is contiguous in memory (or, for the last mode's MTTKRP, its rows
-// are); one shorter than half a chunk would leave most of each step empty, so
-// then it is the longest one.
 }  // namespace
 
-void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner) {
-  int64_t stride[kMaxModes], st = 1;
+// Which contracted mode is the inner one, and the strides of all of them. The
+// inner mode is the fastest contracted one, where a chunk is contiguous in
+// memory (or, for the last mode's MTTKRP, its rows are); one shorter than half a
+// chunk would leave most of each step empty, so then it is the longest one.
+void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner, int cut,
+                   int64_t cut_len) {
+  int64_t stride[kMaxModes], size[kMaxModes], st = 1;
   for (int m = ndim - 1; m >= 0; --m) {
     stride[m] = st;
     st *= shape[m];
+    size[m] = m == cut ? cut_len : shape[m];
   }
   int in = mode == ndim - 1 ? ndim - 2 : ndim - 1;
-  if (shape[in] < VIEW_MIN_RUN)
+  if (size[in] < VIEW_MIN_RUN)
     for (int m = ndim - 1; m >= 0; --m)
-      if (m != mode && shape[m] > shape[in]) in = m;
+      if (m != mode && size[m] > size[in]) in = m;
   *inner = in;
   g->rows = shape[mode];
   g->row_stride = stride[mode];
   g->k_stride = stride[in];
-  g->S = (uint32_t)shape[in];
+  g->S = (uint32_t)size[in];
   int64_t runs = 1;
   for (int m = 0; m < ndim; ++m) {
     if (m == mode || m == in) continue;
-    g->size[g->n_outer] = (uint32_t)shape[m];
+    g->size[g->n_outer] = (uint32_t)size[m];
     g->stride[g->n_outer] = stride[m];
     ++g->n_outer;
-    runs *= shape[m];
+    runs *= size[m];
   }
   // equal chunks of at most 32 columns
   g->chunks = (uint32_t)ceil_div(g->S, 32);

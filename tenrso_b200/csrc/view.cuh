@@ -58,8 +58,10 @@ struct ViewPlan {
 };
 
 // The geometry of one mode's contraction (rows, strides, runs, chunks, outer
-// modes) and its inner mode; element-type independent.
-void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner);
+// modes) and its inner mode; element-type independent. cut >= 0: only `cut_len`
+// indices of the contracted mode `cut` (X and its factor start at the first).
+void describe_view(int ndim, const int64_t* shape, int mode, ViewArgs* g, int* inner,
+                   int cut = -1, int64_t cut_len = 0);
 // The MTTKRP of X (row-major, `shape`) for `mode`, R columns; `reserve`: SMs
 // the plan leaves to other kernels.
 ViewPlan plan_view(const tsr_ctx* ctx, int ndim, const int64_t* shape, int mode, int R,

@@ -95,3 +95,21 @@ def test_f64_calls_give_their_tensor_back():
     assert np.isfinite(res.fit)
     assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
     ctx.close()
+
+
+def test_mttkrp_f64_wide_unfolding():
+    """More columns than 32 bits count: 65537 x 65536 contracted, nonzero on both
+    sides of each piece's ends. One product per term, exact in FP64."""
+    import torch
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 34 GB of device memory")
+    X = np.zeros((1, 65537, 65536))
+    fs = [np.ones((1, 1)), np.arange(65537.0)[:, None] + 1, np.arange(65536.0)[:, None] + 3]
+    want = 0.0
+    for j, k, v in ((0, 0, 1.0), (32767, 5, 2.0), (32768, 65535, -3.0), (65535, 0, 4.0),
+                    (65536, 7, 0.5), (65536, 65535, -1.0)):
+        X[0, j, k] = v
+        want += v * (j + 1) * (k + 3)
+    ctx = tb.Context()
+    assert tb.mttkrp_f64(X, fs, 0, ctx=ctx).tolist() == [[want]]
+    ctx.close()
