@@ -790,8 +790,13 @@ int tsr_mttkrp_all_modes_f32(tsr_ctx* ctx, const float* tensor, int ndim, const 
   std::vector<int64_t> cols(ndim, rank);
   TSR_TRY(validate_mttkrp(ndim, shape, ndim, shape, cols.data(), 0));
   TSR_TRY(check_precision(precision));
+  TSR_TRY(check_sizes(ndim, shape, rank));
   TSR_TRY(check_ctx(ctx));
   const int R = (int)rank;
+  if (numel(ndim, shape) == 0 || R == 0) {  // empty sums: the outputs are zero
+    for (int m = 0; m < ndim; ++m) std::memset(out[m], 0, sizeof(float) * shape[m] * R);
+    return TSR_OK;
+  }
   float* dX = nullptr;
   TSR_TRY(upload_tensor(ctx, tensor, ndim, shape, nullptr, &dX));
   FactorTable ft{};
@@ -841,6 +846,9 @@ int tsr_profile_mttkrp_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim,
   std::vector<int64_t> cols(ndim, rank);
   TSR_TRY(validate_mttkrp(ndim, shape, ndim, shape, cols.data(), mode));
   TSR_TRY(check_precision(precision));
+  TSR_TRY(check_sizes(ndim, shape, rank));
+  if (numel(ndim, shape) == 0 || rank == 0)
+    return fail(TSR_E_INVALID_ARG, "no kernel runs on an empty tensor or rank 0");
   TSR_TRY(check_ctx(ctx));
   FactorTable ft{};
   for (int m = 0; m < ndim; ++m) {

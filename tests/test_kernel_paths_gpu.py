@@ -207,3 +207,15 @@ def test_batched_initial_config(shape, R, expect):
     config = b.config
     b.close()
     assert (config["threads"], config["ctas_per_sm"]) == expect
+
+
+@pytest.mark.parametrize("shape,R", [((4, 0, 3), 2), ((0, 5, 3), 2), ((4, 5, 0), 2), ((4, 5, 3), 0)])
+def test_all_modes_of_an_empty_tensor(shape, R):
+    """Empty sums are zero, for all modes at once as for one."""
+    fs = [np.ones((n, R), np.float32) for n in shape]
+    outs = tb.mttkrp_all_modes(np.ones(shape, np.float32), fs)
+    for m, n in enumerate(shape):
+        assert outs[m].shape == (n, R) and not outs[m].any()
+        assert not tb.mttkrp(np.ones(shape, np.float32), fs, m).any()
+    with pytest.raises(tb.TenrsoError, match="empty tensor"):
+        tb.profile_mttkrp_dev(8, shape, [8, 8, 8], R, 0, "fp32")
