@@ -738,8 +738,8 @@ def run_ours(args):
             "config": {"workload": WORKLOAD, "shape": list(SHAPE), "rank": RANK,
                        "iterations_per_step": ITERS, "precision": "bf16x3",
                        "parallelism": f"replicas{world}" if world > 1 else "1 GPU",
-                       "l2": "working set per step > L2 (X 64 MiB + per-mode unfoldings "
-                             "192 MiB re-written every step)"},
+                       "l2": "working set per step > L2 (X 64 MiB + its bf16 halves 64 MiB "
+                             "re-written every step)"},
             "fp32_path": {"value": fp32_value, "unit": "iter/s", "fit": fit_fp32,
                           "ms_per_step": ms_fp32 / args.steps},
             "speedup_mixed_vs_fp32": value / fp32_value,

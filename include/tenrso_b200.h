@@ -51,8 +51,12 @@ typedef enum tsr_status {
 } tsr_status;
 
 /* Arithmetic of the dense MTTKRP. FP32: IEEE fp32 FMA on the SIMT pipes.
- * BF16X3: operands split as x = hi + lo (both bf16), three tcgen05 bf16 MMAs
- * (hi*hi + hi*lo + lo*hi) with fp32 accumulation in tensor memory. */
+ * BF16X3: operands split as x = hi + lo (both bf16), tcgen05 bf16 MMAs of
+ * hi*hi + hi*lo + lo*hi (and lo*lo in the three-mode form that reads X in its own
+ * layout) with fp32 accumulation in tensor memory. CP-ALS runs the precision it
+ * is given. A single MTTKRP, a reconstruction gradient or an evaluation on a
+ * prepared tensor that asks for BF16X3 may run in FP32, which is more accurate,
+ * where reading X in place is the faster way. */
 typedef enum tsr_precision { TSR_PREC_FP32 = 0, TSR_PREC_BF16X3 = 1 } tsr_precision;
 
 /* cp/types.rs:319-328 ConvergenceReason */
@@ -147,10 +151,12 @@ int tsr_mttkrp_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim, const int6
                        const float* const* d_factors, int64_t rank, int mode, int precision,
                        float* d_out);
 
-/* Kernel-only timing of the dense MTTKRP (the roofline figure): the unfolding
+/* Kernel-only timing of the dense MTTKRP (the roofline figure): the operand
  * is prepared once, then `iters` launches of the MTTKRP kernel are timed with
- * CUDA events on the context's stream, optionally writing a buffer larger
- * than L2 between launches. No tenrso counterpart (measurement aid). */
+ * CUDA events on the context's stream, optionally reading a buffer larger
+ * than L2 between launches. The kernel is the one that CP-ALS runs at `precision`;
+ * a single BF16X3 call may run another (see tsr_precision). An empty tensor or
+ * rank 0 is TSR_E_INVALID_ARG. No tenrso counterpart (measurement aid). */
 int tsr_profile_mttkrp_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim,
                                const int64_t* shape, const float* const* d_factors, int64_t rank,
                                int mode, int precision, int iters, int flush_l2,
@@ -440,8 +446,9 @@ int tsr_cp_residual_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim, const
                             float alpha, float* d_out, double* sq_err);
 /* CpReconstructionGrad::compute_factor_gradients (crates/tenrso-ad/src/grad.rs:81-120),
  * the VjpOp rule of the reconstruction: out_grads[n] (shape[n] x rank) =
- * unfold(G, n) . KR_{m != n}(U_m) . diag(weights), computed as an MTTKRP of G
- * whose Khatri-Rao rows are never stored. Errors as grad.rs:84-91, 137-139. */
+ * unfold(G, n) . KR_{m != n}(U_m) . diag(weights): an MTTKRP of G per mode, or
+ * two contractions of G that every mode's is formed from; Khatri-Rao rows are
+ * never stored. Errors as grad.rs:84-91, 137-139. */
 int tsr_cp_reconstruction_grad_f32(tsr_ctx* ctx, const float* grad_output, int grad_ndim,
                                    const int64_t* shape, const float* const* factors,
                                    int n_factors, const int64_t* factor_rows,
@@ -451,8 +458,9 @@ int tsr_cp_reconstruction_grad_dev_f32(tsr_ctx* ctx, const float* d_grad_output,
                                        const int64_t* shape, const float* const* d_factors,
                                        int64_t rank, const float* d_weights, int precision,
                                        float* const* d_out_grads);
-/* A device tensor prepared for repeated MTTKRPs (no tenrso counterpart): its
- * per-mode unfoldings in `precision` are built once and owned by the object;
+/* A device tensor prepared for repeated MTTKRPs (no tenrso counterpart). FP32
+ * reads d_tensor in place; for BF16X3 its per-mode unfoldings and, where it
+ * suits, a copy in its own layout are built once and owned by the object.
  * d_tensor stays the caller's and must not change while the object lives. */
 typedef struct tsr_dense tsr_dense;
 int tsr_dense_create_dev_f32(tsr_ctx* ctx, const float* d_tensor, int ndim, const int64_t* shape,

@@ -153,8 +153,8 @@ class CpReconstructionOp:
 
 class DenseTensor:
     """A device tensor prepared for repeated MTTKRPs (FP32: read in place;
-    BF16x3: its bf16 form built once). The device buffer at d_tensor must outlive this object and
-    stay unchanged."""
+    BF16x3: its bf16 form built once). The device buffer at d_tensor must
+    outlive this object and stay unchanged."""
 
     def __init__(self, d_tensor: int, shape, precision="fp32", ctx: Optional[Context] = None):
         self.shape = tuple(int(s) for s in shape)

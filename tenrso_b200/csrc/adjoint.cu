@@ -20,7 +20,8 @@
 
 // A dense tensor prepared for repeated MTTKRPs: FP32 reads the tensor in
 // place, BF16x3 keeps what its kernels read (halves in X's own layout, or
-// unfoldings) in HBM. The tensor itself stays the caller's and must not change while the object is in use.
+// unfoldings) in HBM. The tensor itself stays the caller's and must not change
+// while the object is in use.
 struct tsr_dense {
   int ndim = 0;
   int64_t shape[tsr::kMaxModes] = {};

@@ -715,8 +715,9 @@ SmemPlan plan_smem(const tsr_batch* bt, int threads, int ctas_per_sm) {
 // all): one 512-thread CTA per SM, or two of 256. A sweep of an instance of
 // w = n0 n1 n2p (rank padded to 4) takes about 20 us (the solves) + 24 us per
 // 1e6 of w on 512 threads, + 33 us on 256; two CTAs on an SM slow each other's
-// passes by a third (rates from before the load ring of stream_rows, which took
-// a fifth off each). The makespan is that of the largest instance or of the
+// passes by a third. (Rates from before the load ring of stream_rows, which took
+// a fifth off each: of seven batches measured since, from one instance of 64^3
+// to 512 of 16..96, the choice was the faster one in each.) The makespan is that of the largest instance or of the
 // whole batch spread over the slots. Measured: 512 instances of 16..96, 7.6 ms
 // (512 x 1) against 9.2; 300 instances of 8..40, 0.91 against 0.61. Where the SM
 // holds one CTA of 256 only, it is 512: 296 instances of 4 x 5900 x 8 rank 4,

@@ -237,10 +237,10 @@ struct StoreBF16x2 {
 // All unfoldings of a 3-way tensor X[I][J][K] (J, K multiples of 8; rows
 // unpadded) in one pass, plus ||X||^2:
 //   X_(0)[i][j*K + k], X_(1)[j][i*K + k], X_(2)[k][i*J + j]
-// as bf16 hi/lo pairs. A CTA owns a 32 (j) x 64 (k) tile of one slice i: it reads the tile once (128-bit
-// loads), writes modes 0 and 1 as 16-byte row pieces and mode 2 through a
-// shared-memory transpose, 8 consecutive j per thread. Each element's split is
-// formed once for all three copies.
+// as bf16 hi/lo pairs. A CTA owns a 32 (j) x 64 (k) tile of one slice i: it
+// reads the tile once (128-bit loads: X has to be 16-byte aligned), writes modes
+// 0 and 1 as 16-byte row pieces and mode 2 through a shared-memory transpose, 8
+// consecutive j per thread.
 struct Unfold3Out {
   __nv_bfloat16* hi[3];
   __nv_bfloat16* lo[3];

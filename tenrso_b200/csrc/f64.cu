@@ -50,10 +50,12 @@ __device__ __forceinline__ void f64_cp8(double* dst, const double* src, bool ok)
                : "memory");
 }
 
-// 4 x 4 outputs per thread (rows ty + 16 i, columns tx + (BN/4) q). Bound by
-// shared-memory reads (two 8-byte words per two FMAs at 4 x 4). The former
-// kernel divided a 64-bit index per element and multiplied 64 columns whatever
-// the rank: 36 us per mode at 120x100x80 rank 24.
+// 4 x 4 outputs per thread (rows ty + 16 i, columns tx + (BN/4) q): eight 8-byte
+// words read from shared memory per 16 FMAs, which for a warp are about eight
+// wavefronts against eight cycles of FP64 issue. At 120x100x80 rank 24, 13-21 us
+// per mode where the FMAs need 1.4: too few chunks per CTA to hide the loads. The
+// former kernel divided a 64-bit index per element and multiplied 64 columns
+// whatever the rank: 36 us.
 template <int BN>
 __global__ void __launch_bounds__(4 * BN) mttkrp_f64_kernel(const __grid_constant__ M64Args g) {
   constexpr int TX = BN / 4, NT = 4 * BN, NW = NT / 32;

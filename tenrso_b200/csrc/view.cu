@@ -1,5 +1,5 @@
 // Planning and launch of the view kernels (see view.cuh): the FP32 MTTKRP of
-// every dense entry point.
+// every dense entry point but the allocation-free one, and the n-mode products.
 #include "view.cuh"
 
 #include <algorithm>

@@ -430,8 +430,9 @@ def cp_als_f64(tensor, rank: int, max_iters: int, tol: float, init="random",
 def profile_mttkrp_dev(d_tensor: int, shape, d_factors: Sequence[int], rank: int, mode: int,
                        precision="bf16x3", iters: int = 10, flush_l2: bool = True,
                        ctx: Optional[Context] = None):
-    """Mean milliseconds of one MTTKRP kernel launch (operands prepared once),
-    and the split-K count used. Measurement aid for the roofline figure."""
+    """Mean milliseconds of one launch of the MTTKRP kernel that CP-ALS runs at
+    this precision (operands prepared once), and the split-K count used.
+    Measurement aid for the roofline figure."""
     shp = _i64(shape)
     ptrs = (C.c_void_p * len(d_factors))(*d_factors)
     ms = C.c_double(0)
