@@ -559,20 +559,26 @@ int cp_als_device(tsr_ctx* ctx, const float* dX, const tsr_sparse* sp, int ndim,
     void* pp;
     TSR_TRY(slot_get(ctx, SLOT_PARTIALS, sizeof(float) * pmax, &pp));
     a.partials = (float*)pp;
-    if (fused_unfold) {  // the initial Grams on the aux stream beside it
+    // the initial Grams on the aux stream beside the pass that forms ||X||^2
+    // (with the unfoldings, where the fused unfold applies). Not beside the norm
+    // after bf16 unfoldings: there the Grams of a long factor and the join before
+    // the sweep cost more than they hide (one sweep of 64 x 100000 rank 32 351 us
+    // against 299); FP32 sweeps gain up to 5 us a call from it.
+    const bool beside = fused_unfold || precision == TSR_PREC_FP32;
+    if (beside) {
       TSR_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
       TSR_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev[0], 0));
       TSR_TRY(launch_gram_all(ctx, ctx->aux, ndim, a.ft.ptr, shape, R, a.b.grams));
       TSR_CUDA(cudaEventRecord(ctx->ev[1], ctx->aux));
-      TSR_TRY(launch_unfold3(ctx, dX, shape, uhi, ulo, &a.b.state->xnorm_sq));
-      TSR_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev[1], 0));
-    } else {
-      // one after the other: beside the norm, the Grams of a long factor and the
-      // join before the sweep cost more than they hide (one BF16x3 sweep of 64 x
-      // 100000 rank 32 351 us against 299; FP32 and short factors the same)
-      TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
-      TSR_TRY(launch_gram_all(ctx, ctx->stream, ndim, a.ft.ptr, shape, R, a.b.grams));
     }
+    if (fused_unfold)
+      TSR_TRY(launch_unfold3(ctx, dX, shape, uhi, ulo, &a.b.state->xnorm_sq));
+    else
+      TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
+    if (beside)
+      TSR_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev[1], 0));
+    else
+      TSR_TRY(launch_gram_all(ctx, ctx->stream, ndim, a.ft.ptr, shape, R, a.b.grams));
   }
   if (sp || max_iters <= 0) {
     if (!sp) TSR_TRY(launch_norm_sq(ctx, ctx->stream, dX, n, &a.b.state->xnorm_sq));
